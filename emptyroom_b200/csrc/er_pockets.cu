@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "er_ctx.h"
+#include "er_host.h"
 #include "er_nvtx.h"
 
 namespace er {
@@ -586,7 +587,8 @@ namespace er {
 
 struct AccParams {
     double t[9];
-    int nx, ny, nz;
+    double reach[3];  // 1 / (distance between opposite faces), per axis; inf for a flat cell
+    int n[3];
 };
 
 __device__ __forceinline__ void acc_cart(const double* t, double xf, double yf, double zf,
@@ -596,55 +598,86 @@ __device__ __forceinline__ void acc_cart(const double* t, double xf, double yf, 
     z = __dadd_rn(__dadd_rn(__dmul_rn(t[6], xf), __dmul_rn(t[7], yf)), __dmul_rn(t[8], zf));
 }
 
-__global__ void acc_images_kernel(const double4* __restrict__ atoms, int n, AccParams P,
-                                  double4* __restrict__ img) {
-    const int total = 27 * n;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
-        const int a = q / 27, m = q % 27;
-        const int i = m / 9 - 1, j = (m / 3) % 3 - 1, k = m % 3 - 1;
-        const double4 at = atoms[a];
-        double x, y, z;
-        // src/computegridsheet.h:134-140
-        acc_cart(P.t, __dadd_rn(at.x, (double)i), __dadd_rn(at.y, (double)j),
-                 __dadd_rn(at.z, (double)k), x, y, z);
-        img[q] = make_double4(x, y, z, at.w);
-    }
-}
+// Marks the points that one atom image covers: block (x, y, z) takes image y
+// of atom x, and blocks z share its box. An image covers points whose
+// fractional distance along axis d is at most sigma / width_d, so only the
+// lattice box of that half-width (a thousandth of a spacing wider, far above
+// the rounding of its FP64 bounds) is tested, with the reference's own
+// expressions; the other points cannot pass the test. Every covered point is
+// written by whichever images cover it, all with the same 0. Testing every
+// point against every image took 2.3 ms on a 65 x 63 x 64 grid of a 424-atom
+// cell, 3e9 tests; this makes 2.4e6 in 23 us, most of it the turnover of blocks
+// whose image misses the cell and that end at once (32 us with 256 threads a
+// block; 46 us with a loop over the 27 images in one block, where each miss
+// costs the block its latency).
+constexpr int kAccAxis = 1024;  // axis values held on chip (longer boxes divide per point)
+constexpr int kAccThreads = 128;
 
-__global__ void __launch_bounds__(256) acc_grid_kernel(const double4* __restrict__ img, int nimg,
-                                                       AccParams P, uint8_t* __restrict__ out) {
-    __shared__ double4 tile[512];
-    const int64_t n = (int64_t)P.nx * P.ny * P.nz;
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    double x = 0, y = 0, z = 0;
-    bool live = p < n, overlap = false;
-    if (live) {
-        const int k = (int)(p % P.nz), j = (int)((p / P.nz) % P.ny),
-                  i = (int)(p / ((int64_t)P.ny * P.nz));
-        acc_cart(P.t, __ddiv_rn((double)i, (double)(P.nx - 1)),
-                 __ddiv_rn((double)j, (double)(P.ny - 1)),
-                 __ddiv_rn((double)k, (double)(P.nz - 1)), x, y, z);
+__global__ void __launch_bounds__(kAccThreads) acc_mark_kernel(const double4* __restrict__ atoms,
+                                                       const __grid_constant__ AccParams P,
+                                                       uint8_t* __restrict__ out) {
+    __shared__ double axis[kAccAxis];
+    const double4 at = atoms[blockIdx.x];
+    const double s = sqrt(at.w);
+    if (!(s > 0.0)) return;  // r^2 < 0 holds nowhere
+    const int m = blockIdx.y;
+    const double q[3] = {__dadd_rn(at.x, (double)(m / 9 - 1)),
+                         __dadd_rn(at.y, (double)((m / 3) % 3 - 1)),
+                         __dadd_rn(at.z, (double)(m % 3 - 1))};
+    int lo[3], len[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double nm1 = (double)(P.n[d] - 1), w = s * P.reach[d];
+        const double a = fmax(ceil((q[d] - w) * nm1 - 1e-3), 0.0);
+        const double b = fmin(floor((q[d] + w) * nm1 + 1e-3), nm1);
+        if (!(a <= b)) return;  // the same for the whole block
+        lo[d] = (int)a;
+        len[d] = (int)b - (int)a + 1;
     }
-    for (int base = 0; base < nimg; base += 512) {
-        const int cnt = min(512, nimg - base);
-        __syncthreads();
-        for (int q = threadIdx.x; q < cnt; q += blockDim.x) tile[q] = img[base + q];
-        __syncthreads();
-        if (live && !overlap) {
-            for (int q = 0; q < cnt; ++q) {
-                const double4 w = tile[q];
-                const double dx = __dsub_rn(x, w.x), dy = __dsub_rn(y, w.y),
-                             dz = __dsub_rn(z, w.z);
-                const double r2 =
-                    __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                if (r2 < w.w) {  // src/computegridsheet.h:148
-                    overlap = true;
-                    break;
-                }
-            }
+    double ix, iy, iz;
+    acc_cart(P.t, q[0], q[1], q[2], ix, iy, iz);  // src/computegridsheet.h:134-140
+    const bool table = (int64_t)len[0] + len[1] + len[2] <= kAccAxis;
+    if (table) {
+        for (int e = threadIdx.x; e < len[0] + len[1] + len[2]; e += blockDim.x) {
+            const int d = e < len[0] ? 0 : e < len[0] + len[1] ? 1 : 2;
+            const int k = e - (d > 0 ? len[0] : 0) - (d > 1 ? len[1] : 0);
+            axis[e] = __ddiv_rn((double)(lo[d] + k), (double)(P.n[d] - 1));
         }
+        __syncthreads();
     }
-    if (live) out[p] = overlap ? 0 : 1;
+    const int64_t total = (int64_t)len[0] * len[1] * len[2];
+    for (int64_t c = blockIdx.z * (int64_t)blockDim.x + threadIdx.x; c < total;
+         c += (int64_t)gridDim.z * blockDim.x) {
+        int i, j, k;
+        if (total <= INT32_MAX) {
+            const unsigned u = (unsigned)c, row = u / (unsigned)len[2];
+            k = (int)(u - row * (unsigned)len[2]);
+            i = (int)(row / (unsigned)len[1]);
+            j = (int)(row - (unsigned)i * (unsigned)len[1]);
+        } else {
+            const int64_t row = c / len[2];
+            k = (int)(c - row * len[2]);
+            i = (int)(row / len[1]);
+            j = (int)(row - (int64_t)i * len[1]);
+        }
+        double xf, yf, zf, x, y, z;
+        if (table) {
+            xf = axis[i];
+            yf = axis[len[0] + j];
+            zf = axis[len[0] + len[1] + k];
+        } else {
+            xf = __ddiv_rn((double)(lo[0] + i), (double)(P.n[0] - 1));
+            yf = __ddiv_rn((double)(lo[1] + j), (double)(P.n[1] - 1));
+            zf = __ddiv_rn((double)(lo[2] + k), (double)(P.n[2] - 1));
+        }
+        acc_cart(P.t, xf, yf, zf, x, y, z);
+        const double dx = __dsub_rn(x, ix), dy = __dsub_rn(y, iy), dz = __dsub_rn(z, iz);
+        const double r2 =
+            __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        if (r2 < at.w)  // src/computegridsheet.h:148
+            out[(size_t)(lo[2] + k) + (size_t)(lo[1] + j) * P.n[2] +
+                (size_t)(lo[0] + i) * P.n[1] * P.n[2]] = 0;
+    }
 }
 
 }  // namespace er
@@ -656,21 +689,26 @@ extern "C" int er_accessibility(er_ctx* ctx, int fw_id, int nx, int ny, int nz, 
     const er::FwRecord* f = er::find_fw(ctx, fw_id);
     if (!f) return er::set_error(ctx, ER_ERR_NOT_FOUND, "accessibility: unknown framework id");
     const int64_t n = (int64_t)nx * ny * nz;
-    const int nimg = 27 * f->n_atoms;
-    if (ctx->pocket.lab.ensure(std::max<size_t>((size_t)nimg, 1) * sizeof(double4)) ||
-        ctx->pocket.seg.ensure((size_t)n))
+    cudaStream_t st = ctx->stream;
+    if (ctx->pocket.seg.ensure_on((size_t)n, ctx->pool, st))
         return er::set_error(ctx, ER_ERR_NOMEM, "accessibility: scratch allocation failed");
+    uint8_t* mask = (uint8_t*)ctx->pocket.seg.ptr;
     er::AccParams P;
     for (int k = 0; k < 9; ++k) P.t[k] = f->t[k];
-    P.nx = nx; P.ny = ny; P.nz = nz;
-    cudaStream_t st = ctx->stream;
-    double4* img = (double4*)ctx->pocket.lab.ptr;
-    if (nimg > 0)
-        er::acc_images_kernel<<<std::max(1, std::min((nimg + 255) / 256, ctx->num_sms * 8)), 256,
-                                0, st>>>(f->dev.atom_frac, f->n_atoms, P, img);
-    er::acc_grid_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(img, nimg, P,
-                                                                     (uint8_t*)ctx->pocket.seg.ptr);
-    ER_CUDA(ctx, cudaGetLastError());
+    double w[3];
+    er::perpendicular_widths(f->t, w);
+    for (int d = 0; d < 3; ++d) P.reach[d] = w[d] > 0.0 ? 1.0 / w[d] : INFINITY;
+    P.n[0] = nx; P.n[1] = ny; P.n[2] = nz;
+    ER_CUDA(ctx, cudaMemsetAsync(mask, 1, (size_t)n, st));
+    if (f->n_atoms > 0) {
+        // few atoms share each box among more blocks
+        const unsigned parts =
+            (unsigned)std::max(1, std::min(64, 4 * ctx->num_sms / f->n_atoms));
+        er::acc_mark_kernel<<<dim3((unsigned)f->n_atoms, 27, parts), er::kAccThreads, 0,
+                              st>>>(
+            f->dev.atom_frac, P, mask);
+        ER_CUDA(ctx, cudaGetLastError());
+    }
     ER_CUDA(ctx, cudaMemcpyAsync(out, ctx->pocket.seg.ptr, (size_t)n, cudaMemcpyDeviceToHost, st));
     ER_CUDA(ctx, cudaStreamSynchronize(st));
     return ER_OK;

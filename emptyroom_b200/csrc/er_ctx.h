@@ -72,14 +72,17 @@ struct HenryOut {
     int n_blocked;
 };
 
-// Device scratch of one pocket-blocking run (er_pockets.cu): labels,
-// segments, per-segment flags, scan/link tables, a grid copy, the FP64 grid
-// of er_block_pockets.
+// Scratch of one pocket-blocking run (er_pockets.cu): labels, the face-link
+// set, channel roots, their pinned host copy, the FP64 grid of
+// er_block_pockets, and (when the segment numbers are asked for) the ranks of
+// the roots and the segment of every point.
 struct PocketScratch {
     DevBuf grid, lab, seg, flags, misc, mask;
+    HostBuf host;
     void release() {
         DevBuf* b[] = {&grid, &lab, &seg, &flags, &misc, &mask};
         for (DevBuf* x : b) x->release();
+        host.release();
     }
 };
 

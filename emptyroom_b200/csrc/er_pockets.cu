@@ -6,25 +6,27 @@
 // order, links segments across the three periodic faces, and calls a segment
 // a POCKET unless a walk over those links returns to it in another unit cell.
 // Here:
-//   1. init      label[p] = p for accessible points, -1 otherwise
-//   2. union     lock-free union-find over the -x, -y, -z neighbours, first
-//                inside 4 x 8 x 32-point tiles in shared memory, then across
-//                the tile faces in global memory; a root is always linked to
-//                a smaller root, so every component ends rooted at its
-//                smallest linear index
-//   3. compress  label[p] = root
-//   4. number    roots ranked in index order (device-wide scan) -- the
-//                reference's segment numbers, since its flood fill meets each
-//                segment first at the segment's smallest index
-//   5. faces     links (from = segment at N-1, to = segment at 0, direction),
-//                deduplicated in a device hash set
-//   6. classify  on the host: weighted union-find over the (few) links; a
+//   1. tiles     label of every accessible point = smallest point of its
+//                component inside its 4 x 8 x 32-point tile (runs along k by
+//                warp ballots, then union-find over the runs in shared memory)
+//   2. faces     lock-free union-find across the tile faces; a root is always
+//                linked to a smaller root, so every component ends rooted at
+//                its smallest linear index
+//   3. links     (from = root at N-1, to = root at 0, direction) over the
+//                periodic faces, deduplicated in a device hash set
+//   4. classify  on the host: weighted union-find over the (few) links; a
 //                component is a CHANNEL iff some link contradicts the unit-cell
 //                offsets (a cycle with non-zero net translation, self-links
 //                included) -- the same verdict as the reference's DFS, which
 //                checks every link of the component against a spanning walk
-//   7. block     pocket points -> 1e13 (host double grid) or mask = 1 (device)
+//   5. block     channel roots are marked in the label array; every point
+//                walks to its root: pocket points -> 1e13 (host double grid)
+//                or mask = 1 (device), and the pocket roots are counted
+// The reference numbers segments in the order its flood fill meets them, by
+// smallest index: roots ranked in index order (compress and number), needed
+// only when the caller asks for the numbers.
 #include <math.h>
+#include <string.h>
 
 #include <algorithm>
 #include <vector>
@@ -34,20 +36,6 @@
 #include "er_nvtx.h"
 
 namespace er {
-
-__global__ void cc_init_f64(const double* __restrict__ E, int64_t n, double thr,
-                            int* __restrict__ lab) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x)
-        lab[p] = (E[p] >= thr) ? -1 : (int)p;  // src/pocketblocking.cc:138
-}
-
-__global__ void cc_init_f32(const float* __restrict__ E, int64_t n, double thr,
-                            int* __restrict__ lab) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x)
-        lab[p] = ((double)E[p] >= thr) ? -1 : (int)p;
-}
 
 __device__ __forceinline__ int cc_find(const int* lab, int x) {
     int y = lab[x];
@@ -87,16 +75,22 @@ __device__ __forceinline__ void cc_unite(int* lab, int a, int b) {
 }
 
 // Tiled labelling: a CTA labels one tile of kTI x kTJ x kTK points (k fastest,
-// so a warp reads 32 consecutive points) by union-find in shared memory, then
-// writes each accessible point's label as the global index of its tile-local
-// root. Local indices order like global ones inside a tile, and a tile-local
-// root is the smallest index of its local component, so every label is <= its
-// point and roots point to themselves: a valid state for cc_unite. The unions
-// across tile faces follow in cc_union_faces, after every tile has written
-// (a face union into a tile that had not yet written could be overwritten).
-// Against one grid-wide union pass with global atomics: 0.38 -> 0.26 ms for
-// the device pocket mask of a 129^3 grid (block_pockets_device, host-timed).
-constexpr int kTK = 32, kTJ = 8, kTI = 4, kTile = kTK * kTJ * kTI;
+// so a warp's row is 32 consecutive points). A row's accessible points come as
+// one ballot word; each starts at the first point of its run, which joins the
+// neighbours along k without an atomic, and two neighbouring rows need one
+// union per stretch in which both are accessible. Then each accessible point's
+// label is written as the global index of its tile-local root. Local indices
+// order like global ones inside a tile, and a tile-local root is the smallest
+// index of its local component, so every label is <= its point and roots point
+// to themselves: a valid state for cc_unite. The unions across tile faces
+// follow in cc_union_faces, after every tile has written (a face union into a
+// tile that had not yet written could be overwritten).
+// On a 129^3 grid 18 us against 80 with a union per neighbouring pair of points
+// (and 6 for a pass that wrote the first labels), the face unions 17 against
+// 57; the device mask of that grid takes 93 us a call against 247, which
+// numbered every segment and waited for the host four times.
+constexpr int kTK = 32, kTJ = 8, kTI = 4, kTile = kTK * kTJ * kTI, kTRows = kTI * kTJ;
+static_assert(kTK == 32 && kTJ == 8, "a warp per row of points, 256 threads per layer");
 
 __device__ __forceinline__ int cc_find_s(const int* sl, int x) {
     int y = sl[x];
@@ -121,57 +115,103 @@ __device__ __forceinline__ void cc_unite_s(int* sl, int a, int b) {
     }
 }
 
-__global__ void __launch_bounds__(256) cc_union_tiles(int* __restrict__ lab, int nx, int ny,
-                                                      int nz) {
+template <typename G>
+__global__ void __launch_bounds__(256) cc_label_tiles(const G* __restrict__ E, double thr, int nx,
+                                                      int ny, int nz, int* __restrict__ lab) {
     __shared__ int sl[kTile];
+    __shared__ unsigned open[kTRows];  // accessible points of each row
     const int tk = (nz + kTK - 1) / kTK, tj = (ny + kTJ - 1) / kTJ;
-    const int k0 = (blockIdx.x % tk) * kTK;
-    const int j0 = ((blockIdx.x / tk) % tj) * kTJ;
-    const int i0 = (blockIdx.x / (tk * tj)) * kTI;
-    const int64_t syz = (int64_t)ny * nz;
-    auto gidx = [&](int q, bool& in) -> int64_t {
-        const int lk = q % kTK, lj = (q / kTK) % kTJ, li = q / (kTK * kTJ);
-        const int i = i0 + li, j = j0 + lj, k = k0 + lk;
-        in = i < nx && j < ny && k < nz;
-        return (int64_t)k + (int64_t)j * nz + (int64_t)i * syz;
-    };
-    for (int q = threadIdx.x; q < kTile; q += blockDim.x) {
-        bool in;
-        const int64_t g = gidx(q, in);
-        sl[q] = (in && lab[g] >= 0) ? q : -1;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = (int)(blockIdx.x % tk) * kTK + lane;
+    const int j0 = (int)((blockIdx.x / tk) % tj) * kTJ;
+    const int i0 = (int)(blockIdx.x / (tk * tj)) * kTI;
+    // rows w, w + 8, ... of the tile: all kTI loads in flight together
+    G e[kTI];
+    bool in[kTI];
+#pragma unroll
+    for (int u = 0; u < kTI; ++u) {
+        const int i = i0 + u, j = j0 + w;
+        in[u] = i < nx && j < ny && k < nz;
+        if (in[u]) e[u] = E[(int64_t)k + (int64_t)j * nz + (int64_t)i * ny * nz];
+    }
+#pragma unroll
+    for (int u = 0; u < kTI; ++u) {
+        const int row = u * kTJ + w;
+        const bool acc = in[u] && !((double)e[u] >= thr);  // src/pocketblocking.cc:138
+        const unsigned b = __ballot_sync(0xffffffffu, acc);
+        const unsigned gaps = ~b & ((1u << lane) - 1u);  // blocked points below this one
+        sl[row * kTK + lane] = acc ? row * kTK + (gaps ? 32 - __clz(gaps) : 0) : -1;
+        if (lane == 0) open[row] = b;
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < kTile; q += blockDim.x) {
-        if (sl[q] < 0) continue;
-        const int lk = q % kTK, lj = (q / kTK) % kTJ, li = q / (kTK * kTJ);
-        if (lk > 0 && sl[q - 1] >= 0) cc_unite_s(sl, q, q - 1);
-        if (lj > 0 && sl[q - kTK] >= 0) cc_unite_s(sl, q, q - kTK);
-        if (li > 0 && sl[q - kTK * kTJ] >= 0) cc_unite_s(sl, q, q - kTK * kTJ);
+#pragma unroll
+    for (int u = 0; u < kTI; ++u) {
+        const int row = u * kTJ + w, q = row * kTK + lane;
+        const unsigned bit = 1u << lane;
+        if (w > 0) {
+            const unsigned both = open[row] & open[row - 1];
+            if (both & ~(both << 1) & bit) cc_unite_s(sl, q, q - kTK);
+        }
+        if (u > 0) {
+            const unsigned both = open[row] & open[row - kTJ];
+            if (both & ~(both << 1) & bit) cc_unite_s(sl, q, q - kTK * kTJ);
+        }
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < kTile; q += blockDim.x) {
-        if (sl[q] < 0) continue;
-        bool in;
-        const int64_t g = gidx(q, in);
-        lab[g] = (int)gidx(cc_find_s(sl, q), in);
+#pragma unroll
+    for (int u = 0; u < kTI; ++u) {
+        if (!in[u]) continue;
+        const int q = (u * kTJ + w) * kTK + lane;
+        int l = -1;
+        if (sl[q] >= 0) {
+            const int r = cc_find_s(sl, q);
+            l = (int)((int64_t)(k - lane + r % kTK) + (int64_t)(j0 + (r / kTK) % kTJ) * nz +
+                      (int64_t)(i0 + r / (kTK * kTJ)) * ny * nz);
+        }
+        lab[(int64_t)k + (int64_t)(j0 + w) * nz + (int64_t)(i0 + u) * ny * nz] = l;
     }
 }
 
-// Unions across the lower faces of the tiles (global union-find).
-__global__ void cc_union_faces(int* __restrict__ lab, int nx, int ny, int nz) {
-    const int64_t n = (int64_t)nx * ny * nz;
+// Unions across the lower faces of the tiles (global union-find), one thread
+// per face point. Two neighbours along a face that are accessible on both
+// sides, inside one tile on each, are joined there already: only the first of
+// such a stretch unites.
+__global__ void __launch_bounds__(256) cc_union_faces(int* __restrict__ lab, int nx, int ny,
+                                                      int nz) {
     const int64_t syz = (int64_t)ny * nz;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)(p % nz);
-        const int j = (int)((p / nz) % ny);
-        const int i = (int)(p / syz);
-        const bool fk = k > 0 && k % kTK == 0, fj = j > 0 && j % kTJ == 0;
-        const bool fi = i > 0 && i % kTI == 0;
-        if (!(fk || fj || fi) || lab[p] < 0) continue;
-        if (fk && lab[p - 1] >= 0) cc_unite(lab, (int)p, (int)(p - 1));
-        if (fj && lab[p - nz] >= 0) cc_unite(lab, (int)p, (int)(p - nz));
-        if (fi && lab[p - syz] >= 0) cc_unite(lab, (int)p, (int)(p - syz));
+    const int64_t fi = (int64_t)((nx - 1) / kTI) * syz;             // i = kTI, 2 kTI, ...
+    const int64_t fj = (int64_t)((ny - 1) / kTJ) * nx * nz;         // j = kTJ, ...
+    const int64_t fk = (int64_t)((nz - 1) / kTK) * nx * ny;         // k = kTK, ...
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < fi + fj + fk;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        // fewer than 2^31 points: 32-bit quotients
+        int64_t p, across, along;  // the point, its neighbour's and its stretch's offsets
+        bool first;                // the stretch cannot have begun before this point
+        if (q < fi) {
+            const unsigned i = (unsigned)q / (unsigned)syz, r = (unsigned)q % (unsigned)syz;
+            p = (int64_t)(i + 1) * kTI * syz + r;
+            across = syz;
+            along = 1;
+            first = r % (unsigned)nz % kTK == 0;
+        } else if (q < fi + fj) {
+            const unsigned t = (unsigned)(q - fi), k = t % (unsigned)nz, ij = t / (unsigned)nz;
+            const int64_t i = ij % (unsigned)nx, j = (int64_t)(ij / (unsigned)nx + 1) * kTJ;
+            p = k + j * nz + i * syz;
+            across = nz;
+            along = 1;
+            first = k % kTK == 0;
+        } else {
+            const unsigned t = (unsigned)(q - fi - fj), j = t % (unsigned)ny, ik = t / (unsigned)ny;
+            const int64_t i = ik % (unsigned)nx, k = (int64_t)(ik / (unsigned)nx + 1) * kTK;
+            p = k + j * nz + i * syz;
+            across = 1;
+            along = nz;
+            first = j % kTJ == 0;
+        }
+        if (__ldcg(lab + p) < 0 || __ldcg(lab + p - across) < 0) continue;
+        if (!first && __ldcg(lab + p - along) >= 0 && __ldcg(lab + p - along - across) >= 0)
+            continue;
+        cc_unite(lab, (int)p, (int)(p - across));
     }
 }
 
@@ -288,46 +328,61 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
     return x;
 }
 
-// Face links of src/pocketblocking.cc:277-321, inserted once each into an
-// open-addressing set; new keys are appended to `list`.
-__global__ void cc_face_links(const int* __restrict__ seg, int nx, int ny, int nz,
-                              unsigned long long* __restrict__ table, int table_mask,
-                              unsigned long long* __restrict__ list, int* __restrict__ n_list,
-                              int list_cap) {
+// Counters at the head of PocketScratch::misc; the whole block starts as ~0,
+// so each counts from -1.
+struct PocketCounters {
+    int links, pockets;
+};
+constexpr size_t kCounterBytes = 256;
+
+__host__ __device__ inline unsigned long long link_key(int from, int to, int dir) {
+    return ((unsigned long long)from << 33) | ((unsigned long long)to << 2) |
+           (unsigned long long)dir;
+}
+
+// Face links of src/pocketblocking.cc:277-321 between component roots, inserted
+// once each into an open-addressing set; new keys are appended to `list`. A
+// link that the lane before has too is left to it.
+__global__ void __launch_bounds__(256) cc_face_links(const int* __restrict__ lab, int nx, int ny,
+                                                     int nz, unsigned long long* __restrict__ table,
+                                                     int table_mask,
+                                                     unsigned long long* __restrict__ list,
+                                                     int list_cap, PocketCounters* cnt) {
     const int64_t fx = (int64_t)ny * nz, fy = (int64_t)nx * nz, fz = (int64_t)nx * ny;
     const int64_t total = fx + fy + fz;
     const int64_t syz = (int64_t)ny * nz;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        int64_t a, b;
-        int dir;
-        if (q < fx) {  // i = 0 face against i = N_x - 1
-            const int j = (int)(q / nz), k = (int)(q % nz);
-            a = (int64_t)k + (int64_t)j * nz;
-            b = a + (int64_t)(nx - 1) * syz;
-            dir = 1;
-        } else if (q < fx + fy) {  // j = 0 face against j = N_y - 1
-            const int64_t r = q - fx;
-            const int i = (int)(r / nz), k = (int)(r % nz);
-            a = (int64_t)k + (int64_t)i * syz;
-            b = a + (int64_t)(ny - 1) * nz;
-            dir = 2;
-        } else {  // k = 0 face against k = N_z - 1
-            const int64_t r = q - fx - fy;
-            const int i = (int)(r / ny), j = (int)(r % ny);
-            a = (int64_t)j * nz + (int64_t)i * syz;
-            b = a + (nz - 1);
-            dir = 3;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t q0 = blockIdx.x * (int64_t)blockDim.x; q0 < total; q0 += stride) {
+        const int64_t q = q0 + threadIdx.x;
+        unsigned long long key = ~0ull;
+        if (q < total) {
+            int64_t a, b;
+            int dir;
+            if (q < fx) {  // i = 0 face against i = N_x - 1
+                a = q;
+                b = a + (int64_t)(nx - 1) * syz;
+                dir = 1;
+            } else if (q < fx + fy) {  // j = 0 face against j = N_y - 1
+                const unsigned r = (unsigned)(q - fx);
+                a = r % (unsigned)nz + r / (unsigned)nz * syz;
+                b = a + (int64_t)(ny - 1) * nz;
+                dir = 2;
+            } else {  // k = 0 face against k = N_z - 1
+                const unsigned r = (unsigned)(q - fx - fy);
+                a = (int64_t)(r % (unsigned)ny) * nz + r / (unsigned)ny * syz;
+                b = a + (nz - 1);
+                dir = 3;
+            }
+            if (lab[a] >= 0 && lab[b] >= 0)
+                key = link_key(cc_find(lab, (int)b), cc_find(lab, (int)a), dir);
         }
-        const int to = seg[a], from = seg[b];
-        if (to < 0 || from < 0) continue;
-        const unsigned long long key = ((unsigned long long)from << 34) |
-                                       ((unsigned long long)to << 4) | (unsigned long long)dir;
+        const unsigned long long before = __shfl_up_sync(0xffffffffu, key, 1);
+        if (key == ~0ull || ((threadIdx.x & 31) && before == key)) continue;
         unsigned h = (unsigned)(mix64(key) & (uint64_t)table_mask);
         for (int probe = 0; probe <= table_mask; ++probe) {
             const unsigned long long old = atomicCAS(&table[h], ~0ull, key);
             if (old == ~0ull) {
-                const int at = atomicAdd(n_list, 1);
+                const int at = atomicAdd(&cnt->links, 1) + 1;
                 if (at < list_cap) list[at] = key;
                 break;
             }
@@ -337,32 +392,61 @@ __global__ void cc_face_links(const int* __restrict__ seg, int nx, int ny, int n
     }
 }
 
-__global__ void cc_block_f64(double* __restrict__ E, const int* __restrict__ seg, int64_t n,
-                             const unsigned char* __restrict__ pocket) {
+// Channel roots r become -2 - r: the walk to a root ends at any negative label.
+__global__ void cc_mark_channels(const int* __restrict__ roots, int n, int* __restrict__ lab) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) lab[roots[t]] = -2 - roots[t];
+}
+
+// Walks every point to its root. FP64 grid: pocket points become 1e13
+// (src/pocketblocking.cc:373-382); mask: 1 on pocket points, else 0. Counts
+// the pockets (roots that no channel marking reached).
+template <bool MASK>
+__global__ void __launch_bounds__(256) cc_block(const int* __restrict__ lab, int64_t n,
+                                                double* __restrict__ E,
+                                                uint8_t* __restrict__ mask, PocketCounters* cnt) {
+    int roots = 0;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
          p += (int64_t)gridDim.x * blockDim.x) {
-        const int s = seg[p];
-        if (s >= 0 && pocket[s]) E[p] = 1e13;  // src/pocketblocking.cc:373-382
+        int x = (int)p, l = lab[p];
+        roots += l == x;
+        while (l >= 0 && l != x) {
+            x = l;
+            l = lab[x];
+        }
+        if (MASK) mask[p] = l >= 0;
+        else if (l >= 0) E[p] = 1e13;
+    }
+    roots = __reduce_add_sync(0xffffffffu, roots);
+    __shared__ int warp_roots[8];
+    if ((threadIdx.x & 31) == 0) warp_roots[threadIdx.x >> 5] = roots;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int t = 0;
+        for (int k = 0; k < 8; ++k) t += warp_roots[k];
+        if (t) atomicAdd(&cnt->pockets, t);
     }
 }
 
-__global__ void cc_block_mask(uint8_t* __restrict__ mask, const int* __restrict__ seg, int64_t n,
-                              const unsigned char* __restrict__ pocket) {
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int s = seg[p];
-        mask[p] = (s >= 0 && pocket[s]) ? 1 : 0;
+// Host: weighted union-find over the links; the roots of components that have
+// a link which contradicts the unit-cell offsets.
+static std::vector<int> channel_roots(const std::vector<unsigned long long>& links) {
+    std::vector<int> roots;  // every root that has a link, ascending
+    roots.reserve(2 * links.size());
+    for (unsigned long long key : links) {
+        roots.push_back((int)(key >> 33));
+        roots.push_back((int)((key >> 2) & 0x7fffffffull));
     }
-}
-
-// Host: weighted union-find over the links; pocket[s] = 1 unless s's
-// component has a link that contradicts the unit-cell offsets.
-static int classify_segments(int n_seg, const std::vector<unsigned long long>& links,
-                             std::vector<unsigned char>& pocket) {
-    std::vector<int> parent(n_seg);
-    std::vector<int> ox(n_seg, 0), oy(n_seg, 0), oz(n_seg, 0);  // offset to parent
-    std::vector<unsigned char> bad(n_seg, 0);
-    for (int s = 0; s < n_seg; ++s) parent[s] = s;
+    std::sort(roots.begin(), roots.end());
+    roots.erase(std::unique(roots.begin(), roots.end()), roots.end());
+    const int n = (int)roots.size();
+    auto id = [&](int root) {
+        return (int)(std::lower_bound(roots.begin(), roots.end(), root) - roots.begin());
+    };
+    std::vector<int> parent(n);
+    std::vector<int> ox(n, 0), oy(n, 0), oz(n, 0);  // offset to parent
+    std::vector<unsigned char> bad(n, 0);
+    for (int s = 0; s < n; ++s) parent[s] = s;
     auto find = [&](int s, int& x, int& y, int& z) {
         // returns the root and the offset of s relative to it; compresses
         int r = s;
@@ -382,10 +466,8 @@ static int classify_segments(int n_seg, const std::vector<unsigned long long>& l
         return r;
     };
     for (unsigned long long key : links) {
-        const int dir = (int)(key & 15ull);
-        const int to = (int)((key >> 4) & ((1ull << 30) - 1));
-        const int from = (int)(key >> 34);
-        if (from >= n_seg || to >= n_seg || dir < 1 || dir > 3) return -1;
+        const int dir = (int)(key & 3ull);
+        const int to = id((int)((key >> 2) & 0x7fffffffull)), from = id((int)(key >> 33));
         // uc(to) - uc(from) = e_dir (src/pocketblocking.cc:62-83)
         const int ex = dir == 1, ey = dir == 2, ez = dir == 3;
         int fx, fy, fz, tx, ty, tz;
@@ -401,102 +483,119 @@ static int classify_segments(int n_seg, const std::vector<unsigned long long>& l
             bad[rf] |= bad[rt];
         }
     }
-    pocket.assign(n_seg, 0);
-    int n_pockets = 0;
-    for (int s = 0; s < n_seg; ++s) {
+    std::vector<int> out;
+    for (int s = 0; s < n; ++s) {
         int x, y, z;
-        const int r = find(s, x, y, z);
-        pocket[s] = bad[r] ? 0 : 1;
-        n_pockets += pocket[s];
+        if (bad[find(s, x, y, z)]) out.push_back(roots[s]);
     }
-    return n_pockets;
+    return out;
 }
 
-// Steps 2-6 on a labelled grid (ps.lab), on stream st; fills ps.seg (segment
-// per point) and ps.flags (pocket flag per segment, device) and returns the
-// pocket count.
-static int segment_and_classify(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, int nx, int ny,
-                                int nz, int* n_pockets) {
-    const int64_t n = (int64_t)nx * ny * nz;
-    int* lab = (int*)ps.lab.ptr;
-    int* seg = (int*)ps.seg.ptr;
-    const int gb = std::max(1, std::min<int>((int)((n + 255) / 256), ctx->num_sms * 16));
-    {
-        const int64_t tiles = (int64_t)((nz + kTK - 1) / kTK) * ((ny + kTJ - 1) / kTJ) *
-                              ((nx + kTI - 1) / kTI);
-        if (tiles > INT32_MAX) return set_error(ctx, ER_ERR_LIMIT, "pockets: grid too large");
-        cc_union_tiles<<<(unsigned)tiles, 256, 0, st>>>(lab, nx, ny, nz);
-        cc_union_faces<<<gb, 256, 0, st>>>(lab, nx, ny, nz);
+// Sizes of the face-link set and of the scratch that holds it: the counters,
+// the list of links and the hash table, in this order.
+struct LinkLayout {
+    int64_t faces, slots;
+    size_t list_at, table_at, bytes;
+    LinkLayout(int nx, int ny, int nz) {
+        faces = (int64_t)ny * nz + (int64_t)nx * nz + (int64_t)nx * ny;
+        slots = 1024;
+        while (slots < 2 * faces) slots <<= 1;
+        list_at = kCounterBytes;
+        table_at = list_at + (size_t)faces * sizeof(unsigned long long);
+        bytes = table_at + (size_t)slots * sizeof(unsigned long long);
     }
-    cc_compress<<<gb, 256, 0, st>>>(lab, n);
-    const int nblk = (int)((n + kScanItems - 1) / kScanItems);
-    // p_misc: block counts (nblk) | block offsets (nblk + 1) | link count | table | list
-    int* bcount = (int*)ps.misc.ptr;
-    int* boff = bcount + nblk;
-    int* nlink = boff + nblk + 1;
-    cc_root_counts<<<nblk, 1024, 0, st>>>(lab, n, bcount);
-    cc_scan_small<<<1, 1024, 0, st>>>(bcount, boff, nblk);
-    int* rank = (int*)ps.grid.ptr;  // reuse: ranks live only until cc_segments
-    cc_root_ranks<<<nblk, 1024, 0, st>>>(lab, n, boff, rank);
-    cc_segments<<<gb, 256, 0, st>>>(lab, rank, n, seg);
+};
+// Links copied back with their count, before it is known (the others follow).
+constexpr int64_t kFirstLinks = 2048;
+
+// Labels the grid E (device), finds the channels and marks their roots in
+// ps.lab, on stream st, which it synchronises once (twice past kFirstLinks
+// links). With `numbers` the segment of every point goes to ps.seg.
+template <typename G>
+static int label_and_classify(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, const G* E,
+                              double thr, int nx, int ny, int nz, bool numbers) {
+    const int64_t n = (int64_t)nx * ny * nz;
+    const LinkLayout L(nx, ny, nz);
+    const int64_t tiles = (int64_t)((nz + kTK - 1) / kTK) * ((ny + kTJ - 1) / kTJ) *
+                          ((nx + kTI - 1) / kTI);
+    if (tiles > INT32_MAX) return set_error(ctx, ER_ERR_LIMIT, "pockets: grid too large");
+    int* lab = (int*)ps.lab.ptr;
+    char* misc = (char*)ps.misc.ptr;
+    PocketCounters* cnt = (PocketCounters*)misc;
+    unsigned long long* list = (unsigned long long*)(misc + L.list_at);
+    unsigned long long* table = (unsigned long long*)(misc + L.table_at);
+    ER_CUDA(ctx, cudaMemsetAsync(misc, 0xff, L.bytes, st));
+    cc_label_tiles<G><<<(unsigned)tiles, 256, 0, st>>>(E, thr, nx, ny, nz, lab);
+    const int64_t inner = (int64_t)((nx - 1) / kTI) * ny * nz +
+                          (int64_t)((ny - 1) / kTJ) * nx * nz + (int64_t)((nz - 1) / kTK) * nx * ny;
+    auto blocks = [&](int64_t threads) {
+        return (int)std::max<int64_t>(
+            1, std::min<int64_t>((threads + 255) / 256, (int64_t)ctx->num_sms * 32));
+    };
+    if (inner > 0) cc_union_faces<<<blocks(inner), 256, 0, st>>>(lab, nx, ny, nz);
+    cc_face_links<<<blocks(L.faces), 256, 0, st>>>(lab, nx, ny, nz, table, (int)(L.slots - 1), list,
+                                                   (int)L.faces, cnt);
     ER_CUDA(ctx, cudaGetLastError());
-    int n_seg = 0;
-    ER_CUDA(ctx, cudaMemcpyAsync(&n_seg, boff + nblk, sizeof(int), cudaMemcpyDeviceToHost, st));
-    // face links
-    const int64_t faces = (int64_t)ny * nz + (int64_t)nx * nz + (int64_t)nx * ny;
-    int64_t tsize = 1024;
-    while (tsize < 2 * faces) tsize <<= 1;
-    const size_t misc_ints = (size_t)(2 * nblk + 2);
-    const size_t tab_off = ((misc_ints * sizeof(int) + 255) / 256) * 256;
-    unsigned long long* table = (unsigned long long*)((char*)ps.misc.ptr + tab_off);
-    unsigned long long* list = table + tsize;
-    ER_CUDA(ctx, cudaMemsetAsync(table, 0xff, tsize * sizeof(unsigned long long), st));
-    ER_CUDA(ctx, cudaMemsetAsync(nlink, 0, sizeof(int), st));
-    const int fb = std::max(1, std::min<int>((int)((faces + 255) / 256), ctx->num_sms * 8));
-    cc_face_links<<<fb, 256, 0, st>>>(seg, nx, ny, nz, table, (int)(tsize - 1), list, nlink,
-                                      (int)faces);
-    ER_CUDA(ctx, cudaGetLastError());
-    int nl = 0;
-    ER_CUDA(ctx, cudaMemcpyAsync(&nl, nlink, sizeof(int), cudaMemcpyDeviceToHost, st));
+    const int64_t first = std::min(L.faces, kFirstLinks);
+    const size_t head = L.list_at + (size_t)first * sizeof(unsigned long long);
+    ER_CUDA(ctx, cudaMemcpyAsync(ps.host.ptr, misc, head, cudaMemcpyDeviceToHost, st));
+    if (numbers) {
+        const int nblk = (int)((n + kScanItems - 1) / kScanItems);
+        int* rank = (int*)ps.grid.ptr;
+        int* bcount = rank + n;
+        int* boff = bcount + nblk;
+        cc_compress<<<blocks(n), 256, 0, st>>>(lab, n);
+        cc_root_counts<<<nblk, 1024, 0, st>>>(lab, n, bcount);
+        cc_scan_small<<<1, 1024, 0, st>>>(bcount, boff, nblk);
+        cc_root_ranks<<<nblk, 1024, 0, st>>>(lab, n, boff, rank);
+        cc_segments<<<blocks(n), 256, 0, st>>>(lab, rank, n, (int*)ps.seg.ptr);
+        ER_CUDA(ctx, cudaGetLastError());
+    }
     ER_CUDA(ctx, cudaStreamSynchronize(st));
-    std::vector<unsigned long long> links(nl);
-    if (nl) {
-        ER_CUDA(ctx, cudaMemcpyAsync(links.data(), list, nl * sizeof(unsigned long long),
+    const char* h = (const char*)ps.host.ptr;
+    const int nl = ((const PocketCounters*)h)->links + 1;
+    const unsigned long long* hl = (const unsigned long long*)(h + L.list_at);
+    std::vector<unsigned long long> links(hl, hl + std::min<int64_t>(nl, first));
+    if (nl > first) {
+        links.resize(nl);
+        ER_CUDA(ctx, cudaMemcpyAsync(links.data() + first, list + first,
+                                     (size_t)(nl - first) * sizeof(unsigned long long),
                                      cudaMemcpyDeviceToHost, st));
         ER_CUDA(ctx, cudaStreamSynchronize(st));
     }
     // a fixed order makes the host pass independent of the insertion order
     std::sort(links.begin(), links.end());
-    std::vector<unsigned char> pocket;
-    const int np = classify_segments(n_seg, links, pocket);
-    if (np < 0) return set_error(ctx, ER_ERR_INVALID, "pockets: malformed face link");
-    if (ps.flags.ensure_on(std::max<size_t>(pocket.size(), 1), ctx->pool, st) != ER_OK)
-        return set_error(ctx, ER_ERR_NOMEM, "pockets: flag allocation");
-    if (!pocket.empty()) {
-        ER_CUDA(ctx, cudaMemcpyAsync(ps.flags.ptr, pocket.data(), pocket.size(),
-                                     cudaMemcpyHostToDevice, st));
-        ER_CUDA(ctx, cudaStreamSynchronize(st));  // `pocket` is freed on return
+    const std::vector<int> channels = channel_roots(links);
+    if (!channels.empty()) {
+        const size_t bytes = channels.size() * sizeof(int);
+        if (ps.host.ensure(bytes) != ER_OK || ps.flags.ensure_on(bytes, ctx->pool, st) != ER_OK)
+            return set_error(ctx, ER_ERR_NOMEM, "pockets: channel list allocation");
+        memcpy(ps.host.ptr, channels.data(), bytes);  // nothing on st uses it any more
+        ER_CUDA(ctx, cudaMemcpyAsync(ps.flags.ptr, ps.host.ptr, bytes, cudaMemcpyHostToDevice, st));
+        cc_mark_channels<<<(unsigned)((channels.size() + 255) / 256), 256, 0, st>>>(
+            (const int*)ps.flags.ptr, (int)channels.size(), lab);
+        ER_CUDA(ctx, cudaGetLastError());
     }
-    *n_pockets = np;
     return ER_OK;
 }
 
 static int ensure_pocket_scratch(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, int nx, int ny,
-                                 int nz, size_t grid_bytes) {
+                                 int nz, bool numbers) {
     const int64_t n = (int64_t)nx * ny * nz;
-    const int64_t faces = (int64_t)ny * nz + (int64_t)nx * nz + (int64_t)nx * ny;
-    int64_t tsize = 1024;
-    while (tsize < 2 * faces) tsize <<= 1;
-    const int nblk = (int)((n + kScanItems - 1) / kScanItems);
-    const size_t misc_ints = (size_t)(2 * nblk + 2);
-    const size_t tab_off = ((misc_ints * sizeof(int) + 255) / 256) * 256;
-    const size_t misc = tab_off + (size_t)(tsize + faces) * sizeof(unsigned long long);
+    const LinkLayout L(nx, ny, nz);
+    const size_t nblk = (size_t)((n + kScanItems - 1) / kScanItems);
+    const size_t host = L.list_at + (size_t)std::min(L.faces, kFirstLinks) * sizeof(uint64_t);
     cudaMemPool_t pool = ctx->pool;
-    if (ps.lab.ensure_on(n * sizeof(int), pool, st) || ps.seg.ensure_on(n * sizeof(int), pool, st) ||
-        ps.grid.ensure_on(std::max<size_t>(grid_bytes, n * sizeof(int)), pool, st) ||
-        ps.misc.ensure_on(misc, pool, st))
+    if (ps.lab.ensure_on(n * sizeof(int), pool, st) || ps.misc.ensure_on(L.bytes, pool, st) ||
+        (numbers && (ps.seg.ensure_on(n * sizeof(int), pool, st) ||
+                     ps.grid.ensure_on((n + 2 * nblk + 1) * sizeof(int), pool, st))))
         return set_error(ctx, ER_ERR_NOMEM, "pockets: device scratch allocation failed");
+    if (ps.host.ensure(host)) return set_error(ctx, ER_ERR_NOMEM, "pockets: pinned staging failed");
     return ER_OK;
+}
+
+static int block_grid(er_ctx* ctx, int64_t n) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, ctx->num_sms * 16));
 }
 
 static int check_dims(er_ctx* ctx, int nx, int ny, int nz, double T) {
@@ -521,25 +620,27 @@ extern "C" int er_block_pockets(er_ctx* ctx, double* grid, int nx, int ny, int n
     const int64_t n = (int64_t)nx * ny * nz;
     PocketScratch& ps = ctx->pocket;
     cudaStream_t st = ctx->stream;
-    if ((stt = ensure_pocket_scratch(ctx, ps, st, nx, ny, nz, n * sizeof(double))) != ER_OK)
+    if ((stt = ensure_pocket_scratch(ctx, ps, st, nx, ny, nz, segments_out != nullptr)) != ER_OK)
         return stt;
     if (ps.mask.ensure_on(n * sizeof(double), ctx->pool, st) != ER_OK)
         return set_error(ctx, ER_ERR_NOMEM, "pockets: grid allocation failed");
     double* dE = (double*)ps.mask.ptr;
     ER_CUDA(ctx, cudaMemcpyAsync(dE, grid, n * sizeof(double), cudaMemcpyHostToDevice, st));
-    const int gb = std::max(1, std::min<int>((int)((n + 255) / 256), ctx->num_sms * 16));
-    cc_init_f64<<<gb, 256, 0, st>>>(dE, n, 15.0 * temperature, (int*)ps.lab.ptr);
+    if ((stt = label_and_classify(ctx, ps, st, dE, 15.0 * temperature, nx, ny, nz,
+                                  segments_out != nullptr)) != ER_OK)
+        return stt;
+    PocketCounters* cnt = (PocketCounters*)ps.misc.ptr;
+    cc_block<false><<<block_grid(ctx, n), 256, 0, st>>>((const int*)ps.lab.ptr, n, dE, nullptr,
+                                                        cnt);
     ER_CUDA(ctx, cudaGetLastError());
     int np = 0;
-    if ((stt = segment_and_classify(ctx, ps, st, nx, ny, nz, &np)) != ER_OK) return stt;
-    cc_block_f64<<<gb, 256, 0, st>>>(dE, (const int*)ps.seg.ptr, n,
-                                     (const unsigned char*)ps.flags.ptr);
-    ER_CUDA(ctx, cudaGetLastError());
+    ER_CUDA(ctx, cudaMemcpyAsync(&np, &cnt->pockets, sizeof(int), cudaMemcpyDeviceToHost, st));
     ER_CUDA(ctx, cudaMemcpyAsync(grid, dE, n * sizeof(double), cudaMemcpyDeviceToHost, st));
     if (segments_out)
         ER_CUDA(ctx, cudaMemcpyAsync(segments_out, ps.seg.ptr, n * sizeof(int),
                                      cudaMemcpyDeviceToHost, st));
     ER_CUDA(ctx, cudaStreamSynchronize(st));
+    ++np;  // counted from -1
     *n_pockets = np;
     return ER_OK;
 }
@@ -552,16 +653,18 @@ int block_pockets_device_on(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, con
     int stt = check_dims(ctx, nx, ny, nz, temperature);
     if (stt != ER_OK) return stt;
     const int64_t n = (int64_t)nx * ny * nz;
-    if ((stt = ensure_pocket_scratch(ctx, ps, st, nx, ny, nz, 0)) != ER_OK) return stt;
-    const int gb = std::max(1, std::min<int>((int)((n + 255) / 256), ctx->num_sms * 16));
-    cc_init_f32<<<gb, 256, 0, st>>>(grid, n, 15.0 * temperature, (int*)ps.lab.ptr);
+    if ((stt = ensure_pocket_scratch(ctx, ps, st, nx, ny, nz, false)) != ER_OK) return stt;
+    if ((stt = label_and_classify(ctx, ps, st, grid, 15.0 * temperature, nx, ny, nz, false)) !=
+        ER_OK)
+        return stt;
+    PocketCounters* cnt = (PocketCounters*)ps.misc.ptr;
+    cc_block<true><<<block_grid(ctx, n), 256, 0, st>>>((const int*)ps.lab.ptr, n, nullptr, mask_out,
+                                                       cnt);
     ER_CUDA(ctx, cudaGetLastError());
     int np = 0;
-    if ((stt = segment_and_classify(ctx, ps, st, nx, ny, nz, &np)) != ER_OK) return stt;
-    cc_block_mask<<<gb, 256, 0, st>>>(mask_out, (const int*)ps.seg.ptr, n,
-                                      (const unsigned char*)ps.flags.ptr);
-    ER_CUDA(ctx, cudaGetLastError());
+    ER_CUDA(ctx, cudaMemcpyAsync(&np, &cnt->pockets, sizeof(int), cudaMemcpyDeviceToHost, st));
     ER_CUDA(ctx, cudaStreamSynchronize(st));
+    ++np;  // counted from -1
     *n_pockets = np;
     return ER_OK;
 }

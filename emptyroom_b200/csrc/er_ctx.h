@@ -116,7 +116,7 @@ struct er_ctx {
     cudaMemPool_t pool = nullptr;  // stream-ordered pool (framework blocks, plan queues)
     er::DevBuf task_left;    // per-job bricks left (completion notification)
     int* fault_host = nullptr;  // mapped pinned word a kernel sets when a bounded wait
-    int* fault_dev = nullptr;   // gives up (FwDev::fault of every framework), its device address
+    int* fault_dev = nullptr;   // gives up, and its device address
     int* done_host = nullptr;   // mapped pinned per-job completion flags
     int* done_dev = nullptr;    // the same flags, device address
     size_t done_cap = 0;

@@ -48,6 +48,7 @@ constexpr int kThreads = kWarps * 32;
 // points per thread (P) and the CTA brick are set by the point policy (Tile)
 constexpr int kWJ = 4, kWK = 8;            // lanes of a warp sub-brick along j, k
 constexpr int kPMax = 8;                   // largest P any policy uses
+constexpr int kAxisMax = 2 * (kPMax + kWJ + kWK);  // lattice lines of the largest brick, all axes
 constexpr int kMaxCand = 1024;             // CTA candidate capacity per flush
 constexpr int kRowChunk = kThreads;        // cell rows examined per producer pass
 constexpr int kAccChunk = 64;              // atoms per FP32 partial sum (shell lists,
@@ -90,6 +91,7 @@ struct __align__(32) Cand {
     float c12, c12_, nc6, nc6_;  // C12 (twice), -C6 (twice)
 };
 
+// 74.8 KB: at most (228 KB / 3) - 1 KB, so that three CTAs share an SM.
 struct __align__(32) EngineSmem {
     Cand cand[kMaxCand];                   // CTA candidates
     int cid[kMaxCand];                     // their image indices (FP64 paths)
@@ -99,15 +101,26 @@ struct __align__(32) EngineSmem {
                                            // the cutoff for every point (front) and atoms
                                            // crossing it (back)
     double tot[kPMax][kThreads];           // FP64 per-point sums, [p][thread]
-    int row_beg[kRowChunk];
+    union {
+        int row_beg[kRowChunk];
+        double red[kWarps][6];             // warp boxes of the CTA box, before the producer
+    };
     int row_off[kRowChunk];
-    int warp_tot[kWarps];
-    double red[kWarps][6];
-    double box[6];                         // CTA box (FP64 lo, hi)
+    int wcnt[2][kWarps];                   // warp counts of block_prefix, two in turn
+    double box[6];                         // CTA box (FP64 lo, hi; generic points)
+    double org[3];                         // its centre, the origin of FP32 coordinates
+    float cbox[6];                         // CTA box (local FP32 lo, hi)
     float wbox[kWarps][6];                 // warp boxes (local FP32 lo, hi)
-    int item, task;                        // persistent-queue item and its task
-    unsigned long long mbar[2];            // completion barriers of the staged cell rows
+    double axis[kAxisMax];                 // fractional coordinates of a brick's lattice lines
 };
+
+// The block's EngineSmem, by the shared array itself: a reference handed to an
+// out-of-line function arrives as a generic pointer, and the pair loops then
+// run on generic loads (half again as long in a 32^3 grid).
+__device__ __forceinline__ EngineSmem& engine_smem() {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    return *reinterpret_cast<EngineSmem*>(smem_raw);
+}
 
 // ----------------------------------------------------------- packed FP32x2
 typedef unsigned long long f2_t;
@@ -153,7 +166,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return y;
 }
 
-// ------------------------------------------------ bulk copies (TMA engine)
+// ------------------------------------------------ bounded mbarrier wait
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
@@ -163,17 +176,9 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar) {
 __device__ __forceinline__ void mbar_inval(unsigned long long* bar) {
     asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// the single arrival of a phase, announcing the bytes the phase's copies bring
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-// Waits for the phase of `parity` to complete; false after kMbarSpins polls
-// (a copy that never lands: the caller records the fault instead of hanging).
-constexpr int kMbarSpins = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity,
-                                          int spins = kMbarSpins) {
+// Waits for the phase of `parity` to complete; false after `spins` polls (the
+// caller records the fault instead of hanging).
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, int spins) {
     const unsigned a = smem_u32(bar);
     for (int i = 0; i < spins; ++i) {
         unsigned done;
@@ -187,42 +192,24 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     }
     return false;
 }
-// global -> shared copy of `bytes` (a multiple of 16, both addresses 16-byte
-// aligned) by the bulk-copy engine, completing on `bar`; one CTA, no multicast
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes,
-                                         unsigned long long* bar) {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
 
-// Exclusive block scan of one int per thread; *total gets the block sum.
-__device__ __forceinline__ int block_exscan(int v, int* warp_tot, int* total) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
+// Sum of the warps' counts below this warp's; *total gets the sum of all. One
+// barrier per call: consecutive calls use `buf` 0 and 1 in turn, so a warp
+// writes a buffer again only after the barrier of the call between, which
+// every warp reaches after its reads.
+__device__ __forceinline__ int block_prefix(EngineSmem& s, int buf, int count, int* total) {
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) s.wcnt[buf][w] = count;
+    __syncthreads();
+    int below = 0, all = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
+    for (int k = 0; k < kWarps; ++k) {
+        const int c = s.wcnt[buf][k];
+        below += k < w ? c : 0;
+        all += c;
     }
-    if (lane == 31) warp_tot[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int t = lane < kWarps ? warp_tot[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < kWarps; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        if (lane < kWarps) warp_tot[lane] = t;
-    }
-    __syncthreads();
-    int base = w ? warp_tot[w - 1] : 0;
-    *total = warp_tot[kWarps - 1];
-    __syncthreads();
-    return base + x - v;
+    *total = all;
+    return below;
 }
 
 __device__ __forceinline__ void frac_to_cart(const double* t, double xf, double yf, double zf,
@@ -345,6 +332,15 @@ __device__ __forceinline__ float pair_term(float r2, float c12, float nc6) {
 // Lattice points of one (2P) x 8 x 16 brick of a grid job: warp w owns the
 // P x 4 x 8 sub-brick at ((w & 1) P, ((w >> 1) & 1) 4, (w >> 2) 8); lane l the
 // (j, k) = (l / 8, l % 8) column of it and its P points along i.
+//
+// The brick's fractional coordinates i / (N - 1) (FP64 divisions) are formed
+// once per lattice line, one thread each, in `axis` (shared memory); points
+// are products of the table. The boxes need no reduction over the points: a
+// Cartesian coordinate is a chain of rounded products and sums, each monotone
+// in every fractional coordinate, so its extremes over a product set of
+// lattice lines are its values at corners of the set, bit for bit. With every
+// point forming its own divisions twice and FP64 shuffles for the boxes, this
+// took 11,000 of the 84,000 clocks of a CTA (129^3 grid of a 424-atom cell).
 template <int P_>
 struct GridPolicy {
     static constexpr int kP = P_;
@@ -364,18 +360,28 @@ struct GridPolicy {
         j = j0 + ((w >> 1) & 1) * kWJ + lane / kWK;
         k = k0 + (w >> 2) * kWK + lane % kWK;
     }
+    // One thread per lattice line; the caller synchronises. Lines past the
+    // grid repeat its last one (such points are never stored).
+    __device__ __forceinline__ void fill_axes(int tid) const {
+        if (tid >= kBI + kBJ + kBK) return;
+        double* axis = engine_smem().axis;
+        int i, n;
+        if (tid < kBI) { i = i0 + tid; n = T->nx; }
+        else if (tid < kBI + kBJ) { i = j0 + tid - kBI; n = T->ny; }
+        else { i = k0 + tid - kBI - kBJ; n = T->nz; }
+        // axes 1.0 * i / (N - 1), src/writegrid.cu:122-127
+        axis[tid] = __ddiv_rn((double)min(i, n - 1), (double)(n - 1));
+    }
     // Out-of-range points are clamped onto the lattice (same j, k when only i
     // overshoots, so a lane's points keep sharing y and z) and never stored.
     __device__ __forceinline__ bool point(int w, int lane, int p, double* f) const {
         int i, j, k;
         index(w, lane, p, i, j, k);
-        const bool ok = i < T->nx && j < T->ny && k < T->nz;
-        i = min(i, T->nx - 1); j = min(j, T->ny - 1); k = min(k, T->nz - 1);
-        // axes 1.0 * i / (N - 1), src/writegrid.cu:122-127
-        f[0] = __ddiv_rn((double)i, (double)(T->nx - 1));
-        f[1] = __ddiv_rn((double)j, (double)(T->ny - 1));
-        f[2] = __ddiv_rn((double)k, (double)(T->nz - 1));
-        return ok;
+        const double* axis = engine_smem().axis;
+        f[0] = axis[i - i0];
+        f[1] = axis[kBI + j - j0];
+        f[2] = axis[kBI + kBJ + k - k0];
+        return i < T->nx && j < T->ny && k < T->nz;
     }
     // the point's Cartesian position in the positioning frame r
     __device__ __forceinline__ bool cart(const double* r, int w, int lane, int p, double& x,
@@ -384,6 +390,38 @@ struct GridPolicy {
         const bool ok = point(w, lane, p, f);
         frac_to_cart(r, f[0], f[1], f[2], x, y, z);
         return ok;
+    }
+    // FP64 Cartesian box of the lattice points [bi, bi + ni) x [bj, bj + nj) x
+    // [bk, bk + nk) of the brick that lie on the grid; false when there are none.
+    __device__ __forceinline__ bool box(const double* r, int bi, int ni, int bj, int nj, int bk,
+                                        int nk, double* lo, double* hi) const {
+        const int ei = min(bi + ni, T->nx - i0) - 1, ej = min(bj + nj, T->ny - j0) - 1;
+        const int ek = min(bk + nk, T->nz - k0) - 1;
+        if (ei < bi || ej < bj || ek < bk) return false;
+        const double* axis = engine_smem().axis;
+        const double a[3] = {axis[bi], axis[kBI + bj], axis[kBI + kBJ + bk]};
+        const double b[3] = {axis[ei], axis[kBI + ej], axis[kBI + kBJ + ek]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double* t = r + 3 * d;
+            double l[3], h[3];
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                const double u = __dmul_rn(t[e], a[e]), v = __dmul_rn(t[e], b[e]);
+                l[e] = fmin(u, v);
+                h[e] = fmax(u, v);
+            }
+            lo[d] = __dadd_rn(__dadd_rn(l[0], l[1]), l[2]);
+            hi[d] = __dadd_rn(__dadd_rn(h[0], h[1]), h[2]);
+        }
+        return true;
+    }
+    __device__ __forceinline__ bool cta_box(const double* r, double* lo, double* hi) const {
+        return box(r, 0, kBI, 0, kBJ, 0, kBK, lo, hi);
+    }
+    __device__ __forceinline__ bool warp_box(const double* r, int w, double* lo,
+                                             double* hi) const {
+        return box(r, (w & 1) * kP, kP, ((w >> 1) & 1) * kWJ, kWJ, (w >> 2) * kWK, kWK, lo, hi);
     }
     __device__ __forceinline__ void store(int w, int lane, int p, float e) const {
         int i, j, k;
@@ -484,6 +522,11 @@ __device__ __forceinline__ double& tot_at(EngineSmem& s, int p) {
     return s.tot[p][threadIdx.x];
 }
 
+template <int N>
+struct Int {
+    static constexpr int value = N;
+};
+
 // Folds FP32 chunk sums into FP64 registers.
 template <int M>
 __device__ __forceinline__ void fold_regs(double* acc64, f2_t* acc2) {
@@ -512,9 +555,9 @@ __device__ __forceinline__ void fold_packed(EngineSmem& s, f2_t* acc2) {
 
 __device__ __forceinline__ void cta_centre(const EngineSmem& s, double& o0, double& o1,
                                            double& o2) {
-    o0 = 0.5 * (s.box[0] + s.box[3]);
-    o1 = 0.5 * (s.box[1] + s.box[4]);
-    o2 = 0.5 * (s.box[2] + s.box[5]);
+    o0 = s.org[0];
+    o1 = s.org[1];
+    o2 = s.org[2];
 }
 
 // Lattice inner list: every pair inside the cutoff, packed over point pairs.
@@ -536,9 +579,7 @@ __device__ __forceinline__ void lattice_inner(EngineSmem& s, const unsigned shor
     const float py = L.py[0], pz = L.pz[0];
     const char* cbase = reinterpret_cast<const char*>(s.cand);
     const unsigned* wl32 = reinterpret_cast<const unsigned*>(wl);
-    auto atom = [&](unsigned off) {
-        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(cbase + off);       // x x | y z
-        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(cbase + off + 16);  // C12 | -C6
+    auto atom = [&](const ulonglong2 v0, const ulonglong2 v1) {  // x x | y z, C12 | -C6
         if (PREC == PREC_COUNT) {
 #pragma unroll
             for (int m = 0; m < M; ++m) acc2[m] = f2_add(acc2[m], one2);
@@ -559,6 +600,17 @@ __device__ __forceinline__ void lattice_inner(EngineSmem& s, const unsigned shor
             acc2[m] = f2_fma(u3, f2_fma(v1.x, u3, v1.y), acc2[m]);
         }
     };
+    auto atoms = [&](auto n_, const unsigned* off) {
+        constexpr int N = decltype(n_)::value;
+        ulonglong2 v0[N], v1[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            v0[k] = *reinterpret_cast<const ulonglong2*>(cbase + off[k]);
+            v1[k] = *reinterpret_cast<const ulonglong2*>(cbase + off[k] + 16);
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k) atom(v0[k], v1[k]);
+    };
     int q = 0;
     while (q < n_in) {
         const int qe = kComp ? min(q + kChunk, n_in) : n_in;
@@ -566,29 +618,21 @@ __device__ __forceinline__ void lattice_inner(EngineSmem& s, const unsigned shor
         // more independent chains between the MUFU results (256-framework
         // batch: 350 -> 342 ms against two atoms per iteration)
         for (; q + 7 < qe; q += 8) {  // q is a multiple of 8 here (chunk starts are)
-            const uint4 eight = *reinterpret_cast<const uint4*>(wl32 + (q >> 1));
-            atom(eight.x & 0xffffu);
-            atom(eight.x >> 16);
-            atom(eight.y & 0xffffu);
-            atom(eight.y >> 16);
-            atom(eight.z & 0xffffu);
-            atom(eight.z >> 16);
-            atom(eight.w & 0xffffu);
-            atom(eight.w >> 16);
+            const uint4 e = *reinterpret_cast<const uint4*>(wl32 + (q >> 1));
+            const unsigned o0[4] = {e.x & 0xffffu, e.x >> 16, e.y & 0xffffu, e.y >> 16};
+            const unsigned o1[4] = {e.z & 0xffffu, e.z >> 16, e.w & 0xffffu, e.w >> 16};
+            atoms(Int<4>{}, o0);
+            atoms(Int<4>{}, o1);
         }
         for (; q + 3 < qe; q += 4) {
-            const uint2 four = *reinterpret_cast<const uint2*>(wl32 + (q >> 1));
-            atom(four.x & 0xffffu);
-            atom(four.x >> 16);
-            atom(four.y & 0xffffu);
-            atom(four.y >> 16);
+            const uint2 e = *reinterpret_cast<const uint2*>(wl32 + (q >> 1));
+            const unsigned o[4] = {e.x & 0xffffu, e.x >> 16, e.y & 0xffffu, e.y >> 16};
+            atoms(Int<4>{}, o);
         }
-        for (; q + 1 < qe; q += 2) {  // q is even here: chunks have an even length
-            const unsigned two = wl32[q >> 1];
-            atom(two & 0xffffu);
-            atom(two >> 16);
+        for (; q < qe; ++q) {
+            const unsigned o[1] = {wl[q]};
+            atoms(Int<1>{}, o);
         }
-        if (q < qe) atom(wl[q++]);
         fold_regs<M>(acc64, acc2);
     }
 #pragma unroll
@@ -616,9 +660,8 @@ __device__ __forceinline__ int lattice_shell(EngineSmem& s, const unsigned short
     const char* cbase = reinterpret_cast<const char*>(s.cand);
     // the shell list runs backwards from the end of wl
     const unsigned* wl32 = reinterpret_cast<const unsigned*>(wl);
-    auto atom = [&](unsigned off, int q) {
-        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(cbase + off);       // x x | y z
-        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(cbase + off + 16);  // C12 | -C6
+    // the pair terms of one atom; returns its smallest |r^2 - fl32(rc^2)|
+    auto atom = [&](const ulonglong2 v0, const ulonglong2 v1) {  // x x | y z, C12 | -C6
         float ay, az;
         f2_unpack(v0.y, ay, az);
         const float ss = ss_lattice(py, pz, ay, az);
@@ -641,23 +684,46 @@ __device__ __forceinline__ int lattice_shell(EngineSmem& s, const unsigned short
                 acc2[m] = f2_fma(f2_mul(u3, in), f2_fma(v1.x, u3, v1.y), acc2[m]);
             }
         }
-        if (mn <= win) {  // rare: a pair of this atom sits near the cutoff
-            rec = (rec << 10) | (unsigned)q;
-            ++nrec;
+        return mn;
+    };
+    // N atoms (positions q .. q + N - 1 of the list): one branch for them all
+    auto atoms = [&](auto n_, const unsigned* off, int q) {
+        constexpr int N = decltype(n_)::value;
+        ulonglong2 v0[N], v1[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            v0[k] = *reinterpret_cast<const ulonglong2*>(cbase + off[k]);
+            v1[k] = *reinterpret_cast<const ulonglong2*>(cbase + off[k] + 16);
+        }
+        float mn[N], all = INFINITY;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            mn[k] = atom(v0[k], v1[k]);
+            all = fminf(all, mn[k]);
+        }
+        if (all <= win) {  // rare: a pair of these atoms sits near the cutoff
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (mn[k] <= win) {
+                    rec = (rec << 10) | (unsigned)(q + k);
+                    ++nrec;
+                }
         }
     };
     int q = 0;
     while (q < n_sh) {
         const int qe = kComp ? min(q + kAccChunk, n_sh) : n_sh;
-        for (; q + 1 < qe; q += 2) {
-            // entries q, q+1 sit at wl[K-1-q], wl[K-2-q]: one aligned u32
-            const unsigned two = wl32[(kMaxCand - 2 - q) >> 1];
-            atom(two >> 16, q);
-            atom(two & 0xffffu, q + 1);
+        for (; q + 3 < qe; q += 4) {
+            // entries q .. q + 3 sit at wl[K - 1 - q] .. wl[K - 4 - q]: one aligned
+            // 64-bit load (q is a multiple of 4 here: chunks are)
+            const uint2 four = *reinterpret_cast<const uint2*>(wl32 + ((kMaxCand - 4 - q) >> 1));
+            const unsigned off[4] = {four.y >> 16, four.y & 0xffffu, four.x >> 16,
+                                     four.x & 0xffffu};
+            atoms(Int<4>{}, off, q);
         }
-        if (q < qe) {
-            atom(wl[kMaxCand - 1 - q], q);
-            ++q;
+        for (; q < qe; ++q) {
+            const unsigned off[1] = {wl[kMaxCand - 1 - q]};
+            atoms(Int<1>{}, off, q);
         }
         if (kComp) fold_packed<M>(s, acc2);
     }
@@ -878,11 +944,12 @@ __device__ __forceinline__ int generic_lists(EngineSmem& s, const unsigned short
 // re-examined. Kept out of line: it runs for a few
 // lanes of some warps.
 template <class Pol, int PREC>
-static __device__ __noinline__ void recheck_borderline(EngineSmem& s, const Pol& pol,
-                                                       const FwDev& fw, const CutoffConsts& cc,
-                                                       const unsigned short* wl, int n_sh,
+static __device__ __noinline__ void recheck_borderline(const Pol& pol, const FwDev& fw,
+                                                       const CutoffConsts& cc, int n_sh,
                                                        float win, int nrec, unsigned rec,
                                                        const Lane<Pol, PREC>& L) {
+    EngineSmem& s = engine_smem();
+    const unsigned short* wl = s.wl[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const float rc2f = cc.rc2f;
     const bool all = nrec > kRec;
@@ -917,8 +984,128 @@ static __device__ __noinline__ void recheck_borderline(EngineSmem& s, const Pol&
     }
 }
 
+// Near lists of PREC_NEAR64 in FP64: exact positions (FP64 images and points
+// relative to the CTA centre) and FP64 (C12, C6), n_ni atoms inside the cutoff
+// for every point of the warp and n_ns crossing it. A warp's lanes fetch the
+// data of 32 atoms at once into the warp's (by now consumed) inner / shell
+// list, so the fetch latency -- list entry, image index, image, each a
+// dependent load -- is paid once per 32 atoms instead of once per atom, and
+// every lane reads the atoms back by broadcast. Out of line: its FP64 state
+// stays out of the FP32 loops' registers.
+struct __align__(16) NearAtom {
+    double x, y, z, c12, c6, pad;
+};
+constexpr int kNearStage = 32;
+static_assert(kNearStage * sizeof(NearAtom) <= kMaxCand * sizeof(unsigned short),
+              "the staged atoms fit a warp's list");
+
 template <class Pol, int PREC>
-__device__ __forceinline__ void warp_flush_body(EngineSmem& s, const Pol& pol, const FwDev& fw,
+static __device__ __noinline__ void near_lists(const Pol& pol, const FwDev& fw,
+                                               const CutoffConsts& cc, int n_ni, int n_ns,
+                                               const Lane<Pol, PREC>& L) {
+    constexpr int P = Pol::kP;
+    // lattice lanes take all P points in one pass (dy^2 + dz^2 once per atom);
+    // generic points, with their own y and z each, take passes of 4
+    constexpr int kNearP = Pol::kLattice ? P : (P < 4 ? P : 4);
+    EngineSmem& s = engine_smem();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned short* wn = s.wn[w];
+    NearAtom* st = reinterpret_cast<NearAtom*>(s.wl[w]);
+    const double o0 = s.org[0], o1 = s.org[1], o2 = s.org[2];
+    // list entry q counts from the front (inside) or from the back (crossing)
+    auto stage = [&](int q0, int n, bool back) {
+        __syncwarp();  // the warp is done with the list, or with the atoms staged before
+        const int q = q0 + lane;
+        if (q < n) {
+            const int gid = s.cid[wn[back ? kNearCap - 1 - q : q] >> 5];
+            const Atom64 a = atom64(fw, gid, o0, o1, o2);
+            NearAtom& d = st[lane];
+            *reinterpret_cast<double2*>(&d.x) = make_double2(a.x, a.y);
+            *reinterpret_cast<double2*>(&d.z) = make_double2(a.z, a.c12);
+            d.c6 = a.c6;
+        }
+        __syncwarp();
+    };
+    auto staged = [&](int k) {
+        const double2 u = *reinterpret_cast<const double2*>(&st[k].x);
+        const double2 v = *reinterpret_cast<const double2*>(&st[k].z);
+        return Atom64{u.x, u.y, v.x, v.y, st[k].c6};
+    };
+#pragma unroll 1
+    for (int p0 = 0; p0 < P; p0 += kNearP) {
+        double qx[kNearP], qy[Pol::kLattice ? 1 : kNearP], qz[Pol::kLattice ? 1 : kNearP];
+        double nacc[kNearP];
+#pragma unroll
+        for (int p = 0; p < kNearP; ++p) {
+            double x, y, z;
+            pol.cart(fw.r, w, lane, p0 + p, x, y, z);
+            qx[p] = x - o0;
+            if (!Pol::kLattice || p == 0) {
+                qy[Pol::kLattice ? 0 : p] = y - o1;
+                qz[Pol::kLattice ? 0 : p] = z - o2;
+            }
+            nacc[p] = 0.0;
+        }
+        // atoms inside the cutoff for every point of the warp: no test
+        for (int q0 = 0; q0 < n_ni; q0 += kNearStage) {
+            stage(q0, n_ni, false);
+            const int m = min(kNearStage, n_ni - q0);
+            for (int k = 0; k < m; ++k) {
+                const Atom64 a = staged(k);
+                if (Pol::kLattice) {
+                    const double dy = qy[0] - a.y, dz = qz[0] - a.z;
+                    const double yzc = fma(dz, dz, fma(dy, dy, cc.r2min));
+#pragma unroll
+                    for (int p = 0; p < kNearP; ++p)
+                        nacc[p] = near_acc64(nacc[p], qx[p] - a.x, yzc, a.c12, a.c6);
+                } else {
+#pragma unroll
+                    for (int p = 0; p < kNearP; ++p) {
+                        const double dy = qy[Pol::kLattice ? 0 : p] - a.y;
+                        const double dz = qz[Pol::kLattice ? 0 : p] - a.z;
+                        nacc[p] = near_acc64(nacc[p], qx[p] - a.x,
+                                             fma(dz, dz, fma(dy, dy, cc.r2min)), a.c12, a.c6);
+                    }
+                }
+            }
+        }
+        // atoms crossing the cutoff inside the warp box (boxes wider than
+        // rc - kNearR: coarse grids, sparse Widom bins): the cutoff decided per
+        // pair on the FP64 r^2. It differs from the reference's FP64 r^2 (cell
+        // frame, its own rounding) by far less than 1e-12 rc^2, so outside that
+        // window both decide alike and inside it exact_in_cutoff decides.
+        const double rc2lo = fw.rc2 * (1.0 - 1e-12), rc2hi = fw.rc2 * (1.0 + 1e-12);
+        for (int q0 = 0; q0 < n_ns; q0 += kNearStage) {
+            stage(q0, n_ns, true);
+            const int m = min(kNearStage, n_ns - q0);
+            for (int k = 0; k < m; ++k) {
+                const Atom64 a = staged(k);
+#pragma unroll
+                for (int p = 0; p < kNearP; ++p) {
+                    const double dy = qy[Pol::kLattice ? 0 : p] - a.y;
+                    const double dz = qz[Pol::kLattice ? 0 : p] - a.z;
+                    const double dx = qx[p] - a.x;
+                    const double r2 = fmax(fma(dx, dx, fma(dz, dz, dy * dy)), cc.r2min);
+                    bool inside = r2 < rc2lo;
+                    if (!inside && r2 < rc2hi && (L.vmask & (1u << (p0 + p)))) {
+                        double f[3];
+                        pol.point(w, lane, p0 + p, f);
+                        inside = exact_in_cutoff(fw, f, s.cid[wn[kNearCap - 1 - q0 - k] >> 5],
+                                                 cc.r2min);
+                    }
+                    const double u = rcp64_nr(r2);
+                    const double u3 = u * u * u;
+                    if (inside) nacc[p] = fma(u3, fma(a.c12, u3, -a.c6), nacc[p]);
+                }
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < kNearP; ++p) tot_at(s, p0 + p) += nacc[p];
+    }
+}
+
+template <class Pol, int PREC>
+__device__ __forceinline__ void warp_flush(EngineSmem& s, const Pol& pol, const FwDev& fw,
                                                 const CutoffConsts& cc, int n_cand,
                                                 Lane<Pol, PREC>& L) {
     constexpr int P = Pol::kP;
@@ -1049,171 +1236,66 @@ __device__ __forceinline__ void warp_flush_body(EngineSmem& s, const Pol& pol, c
 
     // --- exact re-decision of borderline shell pairs (rare); lanes without a
     // flagged point idle through it
-    if (nrec > 0) recheck_borderline<Pol, PREC>(s, pol, fw, cc, wl, n_sh, win, nrec, rec, L);
-    // --- near lists in FP64: exact positions (FP64 images and points relative
-    // to the CTA centre) and FP64 (C12, C6). Atom-outer order: one atom's loads
-    // serve kNearP of the lane's points per pass.
-    if (kNear && n_ni + n_ns > 0) {
-        // lattice lanes take all P points in one pass (their FP32 list state is
-        // dead by now, so the FP64 point state fits the 80 registers); generic
-        // points, with their own y and z each, take passes of 4
-        constexpr int kNearP = Pol::kLattice ? P : (P < 4 ? P : 4);
-        double o0, o1, o2;
-        cta_centre(s, o0, o1, o2);
-#pragma unroll 1
-        for (int p0 = 0; p0 < P; p0 += kNearP) {
-            double qx[kNearP], qy[Pol::kLattice ? 1 : kNearP], qz[Pol::kLattice ? 1 : kNearP];
-            double nacc[kNearP];
-#pragma unroll
-            for (int p = 0; p < kNearP; ++p) {
-                double y, z;
-                point64(p0 + p, qx[p], y, z);
-                if (!Pol::kLattice || p == 0) {
-                    qy[Pol::kLattice ? 0 : p] = y;
-                    qz[Pol::kLattice ? 0 : p] = z;
-                }
-                nacc[p] = 0.0;
-            }
-            // atoms inside the cutoff for every point of the warp: no test
-            // Widom points: the next atom's FP64 data is loaded while this one's
-            // terms run (the 128-register Widom kernel has room for it; at the
-            // grid kernels' 80 registers it costs more than it hides)
-            constexpr bool kPrefetch = !Pol::kLattice;
-            Atom64 nxt = (kPrefetch && n_ni > 0) ? atom64(fw, s.cid[wn[0] >> 5], o0, o1, o2)
-                                                 : Atom64{};
-            for (int q = 0; q < n_ni; ++q) {
-                Atom64 a;
-                if (kPrefetch) {
-                    a = nxt;
-                    if (q + 1 < n_ni) nxt = atom64(fw, s.cid[wn[q + 1] >> 5], o0, o1, o2);
-                } else {
-                    a = atom64(fw, s.cid[wn[q] >> 5], o0, o1, o2);
-                }
-                if (Pol::kLattice) {
-                    // a lattice lane's points share y and z: dy^2 + dz^2 once per atom
-                    const double dy = qy[0] - a.y, dz = qz[0] - a.z;
-                    const double yzc = fma(dz, dz, fma(dy, dy, cc.r2min));
-#pragma unroll
-                    for (int p = 0; p < kNearP; ++p)
-                        nacc[p] = near_acc64(nacc[p], qx[p] - a.x, yzc, a.c12, a.c6);
-                } else {
-#pragma unroll
-                    for (int p = 0; p < kNearP; ++p) {
-                        const double dy = qy[p] - a.y, dz = qz[p] - a.z;
-                        nacc[p] = near_acc64(nacc[p], qx[p] - a.x,
-                                             fma(dz, dz, fma(dy, dy, cc.r2min)), a.c12, a.c6);
-                    }
-                }
-            }
-            // atoms crossing the cutoff inside the warp box (boxes wider than
-            // rc - kNearR: coarse grids, sparse Widom bins): the cutoff decided per
-            // pair on the FP64 r^2. It differs from the reference's FP64 r^2 (cell
-            // frame, its own rounding) by far less than 1e-12 rc^2, so outside that
-            // window both decide alike and inside it exact_in_cutoff decides.
-            const double rc2lo = fw.rc2 * (1.0 - 1e-12), rc2hi = fw.rc2 * (1.0 + 1e-12);
-            for (int q = 0; q < n_ns; ++q) {
-                const int gid = s.cid[wn[kNearCap - 1 - q] >> 5];
-                const Atom64 a = atom64(fw, gid, o0, o1, o2);
-#pragma unroll 1
-                for (int p = 0; p < kNearP; ++p) {
-                    if (!(L.vmask & (1u << (p0 + p)))) continue;  // never stored
-                    const double dy = qy[Pol::kLattice ? 0 : p] - a.y;
-                    const double dz = qz[Pol::kLattice ? 0 : p] - a.z;
-                    const double dx = qx[p] - a.x;
-                    const double r2 = fmax(fma(dx, dx, fma(dz, dz, dy * dy)), cc.r2min);
-                    bool inside = r2 < rc2lo;
-                    if (!inside && r2 < rc2hi) {
-                        double f[3];
-                        pol.point(w, lane, p0 + p, f);
-                        inside = exact_in_cutoff(fw, f, gid, cc.r2min);
-                    }
-                    if (inside) {
-                        const double u = rcp64_nr(r2);
-                        const double u3 = u * u * u;
-                        nacc[p] = fma(u3, fma(a.c12, u3, -a.c6), nacc[p]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int p = 0; p < kNearP; ++p) tot_at(s, p0 + p) += nacc[p];
-        }
-    }
-}
-
-// Lattice (grid) flushes run out of line: the producer's loop state (box,
-// cell ranges, counters) is saved once around the call instead of staying
-// live in registers through the pair loops (at the 80-register limit of three
-// CTAs per SM that took the 256-framework batch from 370 to 357 ms). The
-// Widom kernel (128 registers, generic points) is faster with the flush
-// inlined: 1.28 ms per 1e7 insertions against 1.61 ms out of line; out of
-// line at 80 registers and three CTAs per SM (P = 4, 6 or 8) it took
-// 1.42-1.51 ms.
-template <class Pol, int PREC>
-static __device__ __noinline__ void warp_flush_call(EngineSmem& s, const Pol& pol,
-                                                    const FwDev& fw, const CutoffConsts& cc,
-                                                    int n_cand, Lane<Pol, PREC>& L) {
-    warp_flush_body<Pol, PREC>(s, pol, fw, cc, n_cand, L);
+    if (nrec > 0) recheck_borderline<Pol, PREC>(pol, fw, cc, n_sh, win, nrec, rec, L);
+    if (kNear && n_ni + n_ns > 0) near_lists<Pol, PREC>(pol, fw, cc, n_ni, n_ns, L);
 }
 
 template <class Pol, int PREC>
-__device__ __forceinline__ void warp_flush(EngineSmem& s, const Pol& pol, const FwDev& fw,
-                                           const CutoffConsts& cc, int n_cand,
-                                           Lane<Pol, PREC>& L) {
-    if constexpr (Pol::kLattice)
-        warp_flush_call<Pol, PREC>(s, pol, fw, cc, n_cand, L);
-    else
-        warp_flush_body<Pol, PREC>(s, pol, fw, cc, n_cand, L);
-}
-
-template <class Pol, int PREC>
-__device__ void process_cta(EngineSmem& s, const Pol& pol, const FwDev& fw,
-                            const CutoffConsts& cc) {
+__device__ void process_cta(const Pol& pol, const FwDev& fw, const CutoffConsts& cc) {
+    EngineSmem& s = engine_smem();
     constexpr int P = Pol::kP;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     Lane<Pol, PREC> L;
 
-    // 1. the CTA box: FP64 bounding box of the valid points
+    // 1. the CTA box (FP64 bounding box of the valid points), whose centre is
+    // the origin of the FP32 coordinates, and the warp box in them
+    double lo0, lo1, lo2, hi0, hi1, hi2;
     L.vmask = 0;
-    double mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY;
-    double mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
+    if constexpr (Pol::kLattice) {
+        pol.fill_axes(tid);
+        __syncthreads();
+        double lo[3], hi[3];
+        pol.cta_box(fw.r, lo, hi);  // a brick holds at least one point of the grid
+        lo0 = lo[0]; lo1 = lo[1]; lo2 = lo[2];
+        hi0 = hi[0]; hi1 = hi[1]; hi2 = hi[2];
+    } else {
+        double mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY;
+        double mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
 #pragma unroll
-    for (int p = 0; p < P; ++p) {
-        double x, y, z;
-        const bool ok = pol.cart(fw.r, w, lane, p, x, y, z);
-        if (ok) {
-            L.vmask |= 1u << p;
-            mn0 = fmin(mn0, x); mn1 = fmin(mn1, y); mn2 = fmin(mn2, z);
-            mx0 = fmax(mx0, x); mx1 = fmax(mx1, y); mx2 = fmax(mx2, z);
+        for (int p = 0; p < P; ++p) {
+            double x, y, z;
+            if (pol.cart(fw.r, w, lane, p, x, y, z)) {
+                mn0 = fmin(mn0, x); mn1 = fmin(mn1, y); mn2 = fmin(mn2, z);
+                mx0 = fmax(mx0, x); mx1 = fmax(mx1, y); mx2 = fmax(mx2, z);
+            }
         }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mn0 = fmin(mn0, __shfl_xor_sync(0xffffffffu, mn0, o));
-        mn1 = fmin(mn1, __shfl_xor_sync(0xffffffffu, mn1, o));
-        mn2 = fmin(mn2, __shfl_xor_sync(0xffffffffu, mn2, o));
-        mx0 = fmax(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-        mx1 = fmax(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
-        mx2 = fmax(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
+        for (int o = 16; o > 0; o >>= 1) {
+            mn0 = fmin(mn0, __shfl_xor_sync(0xffffffffu, mn0, o));
+            mn1 = fmin(mn1, __shfl_xor_sync(0xffffffffu, mn1, o));
+            mn2 = fmin(mn2, __shfl_xor_sync(0xffffffffu, mn2, o));
+            mx0 = fmax(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+            mx1 = fmax(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+            mx2 = fmax(mx2, __shfl_xor_sync(0xffffffffu, mx2, o));
+        }
+        if (lane == 0) {
+            s.red[w][0] = mn0; s.red[w][1] = mn1; s.red[w][2] = mn2;
+            s.red[w][3] = mx0; s.red[w][4] = mx1; s.red[w][5] = mx2;
+        }
+        __syncthreads();
+        if (tid < 6) {
+            double v = s.red[0][tid];
+            for (int k = 1; k < kWarps; ++k)
+                v = (tid < 3) ? fmin(v, s.red[k][tid]) : fmax(v, s.red[k][tid]);
+            s.box[tid] = v;
+        }
+        __syncthreads();
+        lo0 = s.box[0]; lo1 = s.box[1]; lo2 = s.box[2];
+        hi0 = s.box[3]; hi1 = s.box[4]; hi2 = s.box[5];
+        __syncthreads();
+        if (!(lo0 <= hi0)) return;  // no valid point in this CTA
     }
-    L.warp_live = __any_sync(0xffffffffu, L.vmask != 0);
-    if (lane == 0) {
-        s.red[w][0] = mn0; s.red[w][1] = mn1; s.red[w][2] = mn2;
-        s.red[w][3] = mx0; s.red[w][4] = mx1; s.red[w][5] = mx2;
-    }
-    __syncthreads();
-    if (tid < 6) {
-        double v = s.red[0][tid];
-        for (int k = 1; k < kWarps; ++k)
-            v = (tid < 3) ? fmin(v, s.red[k][tid]) : fmax(v, s.red[k][tid]);
-        s.box[tid] = v;
-    }
-    __syncthreads();
-    const double lo0 = s.box[0], lo1 = s.box[1], lo2 = s.box[2];
-    const double hi0 = s.box[3], hi1 = s.box[4], hi2 = s.box[5];
-    __syncthreads();
-    if (!(lo0 <= hi0)) return;  // no valid point in this CTA
-    double o0, o1, o2;
-    cta_centre(s, o0, o1, o2);
+    const double o0 = 0.5 * (lo0 + hi0), o1 = 0.5 * (lo1 + hi1), o2 = 0.5 * (lo2 + hi2);
     L.bul = borderline_ulps(
         cc.rc, cc.rc2f,
         sqrt((hi0 - lo0) * (hi0 - lo0) + (hi1 - lo1) * (hi1 - lo1) + (hi2 - lo2) * (hi2 - lo2)));
@@ -1226,7 +1308,7 @@ __device__ void process_cta(EngineSmem& s, const Pol& pol, const FwDev& fw,
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             double x, y, z;
-            pol.cart(fw.r, w, lane, p, x, y, z);
+            if (pol.cart(fw.r, w, lane, p, x, y, z)) L.vmask |= 1u << p;
             const float fx = (float)(x - o0), fy = (float)(y - o1), fz = (float)(z - o2);
             L.px[p] = fx;
             if (!Pol::kLattice || p == 0) {
@@ -1234,19 +1316,30 @@ __device__ void process_cta(EngineSmem& s, const Pol& pol, const FwDev& fw,
                 L.pz[Pol::kLattice ? 0 : p] = fz;
             }
             tot_at(s, p) = 0.0;
-            if (L.vmask & (1u << p)) {
+            if (!Pol::kLattice && (L.vmask & (1u << p))) {
                 wl0x = fminf(wl0x, fx); wl0y = fminf(wl0y, fy); wl0z = fminf(wl0z, fz);
                 wh0x = fmaxf(wh0x, fx); wh0y = fmaxf(wh0y, fy); wh0z = fmaxf(wh0z, fz);
             }
         }
+        if constexpr (Pol::kLattice) {
+            // x -> (float)(x - o) is monotone too
+            double lo[3], hi[3];
+            L.warp_live = pol.warp_box(fw.r, w, lo, hi);
+            if (L.warp_live) {
+                wl0x = (float)(lo[0] - o0); wl0y = (float)(lo[1] - o1); wl0z = (float)(lo[2] - o2);
+                wh0x = (float)(hi[0] - o0); wh0y = (float)(hi[1] - o1); wh0z = (float)(hi[2] - o2);
+            }
+        } else {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            wl0x = fminf(wl0x, __shfl_xor_sync(0xffffffffu, wl0x, o));
-            wl0y = fminf(wl0y, __shfl_xor_sync(0xffffffffu, wl0y, o));
-            wl0z = fminf(wl0z, __shfl_xor_sync(0xffffffffu, wl0z, o));
-            wh0x = fmaxf(wh0x, __shfl_xor_sync(0xffffffffu, wh0x, o));
-            wh0y = fmaxf(wh0y, __shfl_xor_sync(0xffffffffu, wh0y, o));
-            wh0z = fmaxf(wh0z, __shfl_xor_sync(0xffffffffu, wh0z, o));
+            for (int o = 16; o > 0; o >>= 1) {
+                wl0x = fminf(wl0x, __shfl_xor_sync(0xffffffffu, wl0x, o));
+                wl0y = fminf(wl0y, __shfl_xor_sync(0xffffffffu, wl0y, o));
+                wl0z = fminf(wl0z, __shfl_xor_sync(0xffffffffu, wl0z, o));
+                wh0x = fmaxf(wh0x, __shfl_xor_sync(0xffffffffu, wh0x, o));
+                wh0y = fmaxf(wh0y, __shfl_xor_sync(0xffffffffu, wh0y, o));
+                wh0z = fmaxf(wh0z, __shfl_xor_sync(0xffffffffu, wh0z, o));
+            }
+            L.warp_live = wl0x <= wh0x;
         }
         if (lane == 0) {
             s.wbox[w][0] = wl0x; s.wbox[w][1] = wl0y; s.wbox[w][2] = wl0z;
@@ -1255,208 +1348,126 @@ __device__ void process_cta(EngineSmem& s, const Pol& pol, const FwDev& fw,
         __syncwarp();
     }
 
-// ER_BULK=1 (a build option: `make -C emptyroom_b200/csrc clean all cli
-// ER_BULK=1`) selects the producer whose cell-row image ranges arrive in
-// shared memory by bulk copies of the TMA engine (cp.async.bulk, 256 images
-// per stage, two stages in flight, each completing on an mbarrier whose wait
-// is bounded). Measured on the 256-framework batch it is slower than the
-// default producer (per-thread loads of the same images): 352.1 against
-// 341.6 ms in the default mode, 305.8 against 297.3 ms in ER_PREC_COMP, a
-// Widom call of 1e7 insertions 1.741 against 1.727 ms -- each stage adds a
-// block-wide wait, and the staging state raises the producer's register
-// spills (grid_persistent_kernel<3>: 364 / 1000 bytes of spill stores / loads
-// against 280 / 584).
-#ifndef ER_BULK
-#define ER_BULK 0
-#endif
-#if ER_BULK
-    // staging barriers of this pass (initialised here, invalidated at its end)
-    if (tid == 0) {
-        mbar_init(&s.mbar[0]);
-        mbar_init(&s.mbar[1]);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-#endif
-#if ER_BULK
-    unsigned mph = 0;    // phase parity of each staging barrier
-#endif
-    bool fault = false;  // a staging wait gave up
-    // 3. producer: rows of cells around the CTA box, streamed into shared memory
-    const double R = cc.rcm, R2 = R * R;
-    const float R2f = (float)R2;
-    const float b0x = (float)(lo0 - o0), b0y = (float)(lo1 - o1), b0z = (float)(lo2 - o2);
-    const float b1x = (float)(hi0 - o0), b1y = (float)(hi1 - o1), b1z = (float)(hi2 - o2);
+    // 3. producer: rows of cells around the CTA box, streamed into shared memory.
+    // What its loops need of the box lies in shared memory: held in registers
+    // it would spill around every flush.
     int c0[3], c1[3];
     {
         const double lov[3] = {lo0, lo1, lo2}, hiv[3] = {hi0, hi1, hi2};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            c0[d] = max(0, (int)floor((lov[d] - R - fw.cell_lo[d]) * fw.inv_h));
-            c1[d] = min(fw.nc[d] - 1, (int)floor((hiv[d] + R - fw.cell_lo[d]) * fw.inv_h));
+            c0[d] = max(0, (int)floor((lov[d] - cc.rcm - fw.cell_lo[d]) * fw.inv_h));
+            c1[d] = min(fw.nc[d] - 1, (int)floor((hiv[d] + cc.rcm - fw.cell_lo[d]) * fw.inv_h));
         }
     }
-    int n_cand = 0;
-    if (c0[0] <= c1[0] && c0[1] <= c1[1] && c0[2] <= c1[2]) {
-        const int nyr = c1[1] - c0[1] + 1, nzr = c1[2] - c0[2] + 1;
-        const int nrows = nyr * nzr;
-        for (int rb = 0; rb < nrows; rb += kRowChunk) {
-            const int r = rb + tid;
-            int beg = 0, len = 0;
-            if (r < nrows) {
-                const int ry = c0[1] + r % nyr, rz = c0[2] + r / nyr;
-                const double ylo = fw.cell_lo[1] + ry * fw.h, yhi = ylo + fw.h;
-                const double zlo = fw.cell_lo[2] + rz * fw.h, zhi = zlo + fw.h;
-                const double dy = fmax(0.0, fmax(ylo - hi1, lo1 - yhi));
-                const double dz = fmax(0.0, fmax(zlo - hi2, lo2 - zhi));
-                const double d2 = dy * dy + dz * dz;
-                if (d2 < R2) {
-                    const double ex = sqrt(R2 - d2);
-                    const int xa = max(c0[0], (int)floor((lo0 - ex - fw.cell_lo[0]) * fw.inv_h));
-                    const int xb = min(c1[0], (int)floor((hi0 + ex - fw.cell_lo[0]) * fw.inv_h));
-                    if (xa <= xb) {
-                        const int rowb = (rz * fw.nc[1] + ry) * fw.nc[0];
-                        beg = fw.cell_start[rowb + xa];
-                        len = fw.cell_start[rowb + xb + 1] - beg;
-                    }
-                }
-            }
-            int tot;
-            const int off = block_exscan(len, s.warp_tot, &tot);
-            s.row_beg[tid] = beg;
-            s.row_off[tid] = off;
-            __syncthreads();
-            const int nr = min(kRowChunk, nrows - rb);
-#if ER_BULK
-            // the rows' image ranges arrive by bulk copies, kThreads images
-            // per stage, two stages in flight in the staging area (the per-warp
-            // lists, unused while the producer runs)
-            double4* stg = reinterpret_cast<double4*>(&s.wl[0][0]);
-            const int nst = (tot + kThreads - 1) / kThreads;
-            auto issue = [&](int k) {
-                const int b = k & 1;
-                const int lo = k * kThreads, hi = min(tot, lo + kThreads);
-                if (tid == 0) mbar_expect_tx(&s.mbar[b], (unsigned)(hi - lo) * 32u);
-                const int a = max(lo, off), e = min(hi, off + len);
-                if (a < e)
-                    bulk_g2s(stg + b * kThreads + (a - lo), fw.img_xyz + beg + (a - off),
-                             (unsigned)(e - a) * 32u, &s.mbar[b]);
-            };
-            if (nst > 0) issue(0);
-            for (int k = 0; k < nst; ++k) {
-                const int b = k & 1;
-                if (k + 1 < nst) issue(k + 1);
-                fault |= !mbar_wait(&s.mbar[b], (mph >> b) & 1u);
-                mph ^= 1u << b;
-                const int c = k * kThreads + tid;
-                int pass = 0, g = 0;
-                float ax = 0.f, ay = 0.f, az = 0.f, c12 = 0.f, nc6 = 0.f;
-                if (c < tot) {
-                    const double4 ap = stg[b * kThreads + tid];
-                    ax = (float)(ap.x - o0);
-                    ay = (float)(ap.y - o1);
-                    az = (float)(ap.z - o2);
-                    const float ddx = fmaxf(0.f, fmaxf(b0x - ax, ax - b1x));
-                    const float ddy = fmaxf(0.f, fmaxf(b0y - ay, ay - b1y));
-                    const float ddz = fmaxf(0.f, fmaxf(b0z - az, az - b1z));
-                    pass = (ddx * ddx + ddy * ddy + ddz * ddz) < R2f;
-                    if (pass) {
-                        int a = 0, bb = nr - 1;
-                        while (a < bb) {
-                            const int mid = (a + bb + 1) >> 1;
-                            if (s.row_off[mid] <= c) a = mid; else bb = mid - 1;
-                        }
-                        g = s.row_beg[a] + (c - s.row_off[a]);
-                        const float2 pr = fw.img_par[g];
-                        c12 = pr.x;
-                        nc6 = pr.y;
-                    }
-                }
-                int npass;
-                const int pos = block_exscan(pass, s.warp_tot, &npass);
-                if (n_cand + npass > kMaxCand) {
-                    // the flush writes the staging area: the next stage lands
-                    // first and is copied again after it
-                    if (k + 1 < nst) {
-                        fault |= !mbar_wait(&s.mbar[b ^ 1], (mph >> (b ^ 1)) & 1u);
-                        mph ^= 1u << (b ^ 1);
-                    }
-                    __syncthreads();
-                    warp_flush<Pol, PREC>(s, pol, fw, cc, n_cand, L);
-                    __syncthreads();
-                    n_cand = 0;
-                    if (k + 1 < nst) issue(k + 1);
-                }
-                if (pass) {
-                    Cand& dst = s.cand[n_cand + pos];
-                    *reinterpret_cast<float4*>(&dst.ax) = make_float4(ax, ax, ay, az);
-                    *reinterpret_cast<float4*>(&dst.c12) = make_float4(c12, c12, nc6, nc6);
-                    s.cid[n_cand + pos] = g;
-                }
-                n_cand += npass;
-            }
-#else
-            for (int cb = 0; cb < tot; cb += kThreads) {
-                const int c = cb + tid;
-                int pass = 0, g = 0;
-                float ax = 0.f, ay = 0.f, az = 0.f, c12 = 0.f, nc6 = 0.f;
-                if (c < tot) {
-                    int a = 0, b = nr - 1;
-                    while (a < b) {
-                        const int mid = (a + b + 1) >> 1;
-                        if (s.row_off[mid] <= c) a = mid; else b = mid - 1;
-                    }
-                    g = s.row_beg[a] + (c - s.row_off[a]);
-                    const double4 ap = fw.img_xyz[g];
-                    ax = (float)(ap.x - o0);
-                    ay = (float)(ap.y - o1);
-                    az = (float)(ap.z - o2);
-                    const float ddx = fmaxf(0.f, fmaxf(b0x - ax, ax - b1x));
-                    const float ddy = fmaxf(0.f, fmaxf(b0y - ay, ay - b1y));
-                    const float ddz = fmaxf(0.f, fmaxf(b0z - az, az - b1z));
-                    pass = (ddx * ddx + ddy * ddy + ddz * ddz) < R2f;
-                    if (pass) {
-                        const float2 pr = fw.img_par[g];
-                        c12 = pr.x;
-                        nc6 = pr.y;
-                    }
-                }
-                int npass;
-                const int pos = block_exscan(pass, s.warp_tot, &npass);
-                if (n_cand + npass > kMaxCand) {
-                    __syncthreads();
-                    warp_flush<Pol, PREC>(s, pol, fw, cc, n_cand, L);
-                    __syncthreads();
-                    n_cand = 0;
-                }
-                if (pass) {
-                    Cand& dst = s.cand[n_cand + pos];
-                    *reinterpret_cast<float4*>(&dst.ax) = make_float4(ax, ax, ay, az);
-                    *reinterpret_cast<float4*>(&dst.c12) = make_float4(c12, c12, nc6, nc6);
-                    s.cid[n_cand + pos] = g;
-                }
-                n_cand += npass;
-            }
-#endif
-            __syncthreads();
-        }
-    }
-    if (n_cand > 0) {
-        __syncthreads();
-        warp_flush<Pol, PREC>(s, pol, fw, cc, n_cand, L);
-    }
-    // 4. store (nothing when a staging wait gave up: the pass is reported
-    // through the fault word instead of storing energies of missing atoms)
-    if (__syncthreads_or(fault)) {
-        if (tid == 0 && fw.fault) atomicExch(fw.fault, 1);
-        L.vmask = 0;
-    }
-#if ER_BULK
     if (tid == 0) {
-        mbar_inval(&s.mbar[0]);
-        mbar_inval(&s.mbar[1]);
+        s.org[0] = o0; s.org[1] = o1; s.org[2] = o2;
+        s.cbox[0] = (float)(lo0 - o0); s.cbox[1] = (float)(lo1 - o1); s.cbox[2] = (float)(lo2 - o2);
+        s.cbox[3] = (float)(hi0 - o0); s.cbox[4] = (float)(hi1 - o1); s.cbox[5] = (float)(hi2 - o2);
     }
-#endif
+    __syncthreads();
+    const float R2f = (float)(cc.rcm * cc.rcm);
+    // rows are pruned in FP32 with a millimetre of slack in a metre: every
+    // image that passes the test below lies in the pruned range
+    const float Rrow = (float)cc.rcm + 1e-3f, R2row = Rrow * Rrow;
+    // Fills the candidate list, flushes it and goes on until every row is done.
+    // One flush site (the pair loops are inlined there), and a chunk of images
+    // that no longer fits is taken again after the flush, so that no thread
+    // holds an image through the pair loops.
+    int nyr = 0, nrows = 0;
+    if (c0[0] <= c1[0] && c0[1] <= c1[1] && c0[2] <= c1[2]) {
+        nyr = c1[1] - c0[1] + 1;
+        nrows = nyr * (c1[2] - c0[2] + 1);
+    }
+    int rb = 0, cb = 0, tot = 0, nr = 0, buf = 0;
+    for (bool more = true; more;) {
+        int n_cand = 0;
+        for (;;) {
+            if (cb >= tot) {  // the next chunk of rows
+                if (rb >= nrows) {
+                    more = false;
+                    break;
+                }
+                const int r = rb + tid;
+                int beg = 0, len = 0;
+                if (r < nrows) {
+                    const int ry = c0[1] + r % nyr, rz = c0[2] + r / nyr;
+                    const float y = (float)(fw.cell_lo[1] + ry * fw.h - s.org[1]);
+                    const float z = (float)(fw.cell_lo[2] + rz * fw.h - s.org[2]);
+                    const float hf = (float)fw.h;
+                    const float dy = fmaxf(0.f, fmaxf(y - s.cbox[4], s.cbox[1] - (y + hf)));
+                    const float dz = fmaxf(0.f, fmaxf(z - s.cbox[5], s.cbox[2] - (z + hf)));
+                    const float d2 = dy * dy + dz * dz;
+                    if (d2 < R2row) {
+                        const float ex = sqrtf(R2row - d2);
+                        const double x0 = s.org[0] - fw.cell_lo[0];
+                        const int xa = max(c0[0], (int)floor((x0 + (s.cbox[0] - ex)) * fw.inv_h));
+                        const int xb = min(c1[0], (int)floor((x0 + (s.cbox[3] + ex)) * fw.inv_h));
+                        if (xa <= xb) {
+                            const int rowb = (rz * fw.nc[1] + ry) * fw.nc[0];
+                            beg = fw.cell_start[rowb + xa];
+                            len = fw.cell_start[rowb + xb + 1] - beg;
+                        }
+                    }
+                }
+                int off = len;  // inclusive scan over the warp
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, off, o);
+                    if (lane >= o) off += v;
+                }
+                off += block_prefix(s, buf, __shfl_sync(0xffffffffu, off, 31), &tot) - len;
+                buf ^= 1;
+                s.row_beg[tid] = beg;
+                s.row_off[tid] = off;
+                __syncthreads();
+                nr = min(kRowChunk, nrows - rb);
+                rb += kRowChunk;
+                cb = 0;
+                continue;
+            }
+            const int c = cb + tid;
+            bool pass = false;
+            int g = 0;
+            float ax = 0.f, ay = 0.f, az = 0.f;
+            float2 pr = make_float2(0.f, 0.f);
+            if (c < tot) {
+                int a = 0, b = nr - 1;
+                while (a < b) {
+                    const int mid = (a + b + 1) >> 1;
+                    if (s.row_off[mid] <= c) a = mid; else b = mid - 1;
+                }
+                g = s.row_beg[a] + (c - s.row_off[a]);
+                const double4 ap = fw.img_xyz[g];
+                pr = fw.img_par[g];
+                ax = (float)(ap.x - s.org[0]);
+                ay = (float)(ap.y - s.org[1]);
+                az = (float)(ap.z - s.org[2]);
+                const float ddx = fmaxf(0.f, fmaxf(s.cbox[0] - ax, ax - s.cbox[3]));
+                const float ddy = fmaxf(0.f, fmaxf(s.cbox[1] - ay, ay - s.cbox[4]));
+                const float ddz = fmaxf(0.f, fmaxf(s.cbox[2] - az, az - s.cbox[5]));
+                pass = (ddx * ddx + ddy * ddy + ddz * ddz) < R2f;
+            }
+            const unsigned ball = __ballot_sync(0xffffffffu, pass);
+            int npass;
+            const int pos = n_cand + __popc(ball & ((1u << lane) - 1u)) +
+                            block_prefix(s, buf, __popc(ball), &npass);
+            buf ^= 1;
+            if (n_cand + npass > kMaxCand) break;
+            if (pass) {
+                Cand& dst = s.cand[pos];
+                *reinterpret_cast<float4*>(&dst.ax) = make_float4(ax, ax, ay, az);
+                *reinterpret_cast<float4*>(&dst.c12) = make_float4(pr.x, pr.x, pr.y, pr.y);
+                s.cid[pos] = g;
+            }
+            n_cand += npass;
+            cb += kThreads;
+        }
+        __syncthreads();
+        if (n_cand > 0) warp_flush<Pol, PREC>(s, pol, fw, cc, n_cand, L);
+        if (more) __syncthreads();
+    }
+    // 4. store
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         if (L.vmask & (1u << p)) {

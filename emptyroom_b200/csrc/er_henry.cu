@@ -377,13 +377,11 @@ __global__ void henry_order_straddling_kernel(const int* __restrict__ starts, in
 template <int P>
 __global__ void __launch_bounds__(kThreads, 2)
     henry_energy_kernel(const __grid_constant__ PointTask task) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
     if ((long long)blockIdx.x * (kWarps * 32 * P) >= (long long)*task.n_valid) return;
-    EngineSmem& s = *reinterpret_cast<EngineSmem*>(smem_raw);
     PointPolicy<P> pol(&task, blockIdx.x);
     // near pairs in FP64: a Boltzmann factor turns an energy error dE into a
     // relative weight error dE / T, so Widom energies get the tighter mode
-    process_cta<PointPolicy<P>, PREC_NEAR64>(s, pol, task.fw, task.cc);
+    process_cta<PointPolicy<P>, PREC_NEAR64>(pol, task.fw, task.cc);
 }
 
 __device__ __forceinline__ Lse lse_merge(Lse a, Lse b) {

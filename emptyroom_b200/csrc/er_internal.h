@@ -32,8 +32,6 @@ struct FwDev {
     double rc2;               // squared cutoff, FP64 (the reference's r_cutoff_squared)
     int rep[3];
     int imgs_per_atom;        // (2 rep0 + 1)(2 rep1 + 1)(2 rep2 + 1)
-    int* fault;               // set to 1 by a kernel whose bounded wait gave up (the
-                              // context's mapped fault word; may be null)
 };
 
 // Per-launch constants derived from the cutoff.
@@ -70,12 +68,6 @@ struct PointTask {
                              // regenerated from it for the exact cutoff decisions)
     const int* n_valid;      // device count of entries in `order`
     float* energies;         // E per insertion (insertion order)
-};
-
-// Persistent-queue item as the kernel decodes it: (task position, brick).
-struct WorkItem {
-    int task;
-    int brick;
 };
 
 }  // namespace er

@@ -136,7 +136,7 @@ typedef struct {
     float* out_device; /* device buffer of nx*ny*nz floats */
 } er_grid_job;
 
-#define ER_BATCH_PERSISTENT 0 /* one persistent launch over a device work queue */
+#define ER_BATCH_PERSISTENT 0 /* one launch over a device work queue */
 #define ER_BATCH_PLAIN 1      /* one plain launch per job, in order */
 #define ER_BATCH_HOST_OUT 0x100 /* or-ed into mode: out_device fields are host pointers;
                                    grids are staged on the device and copied back */
@@ -469,9 +469,8 @@ int er_probe_rcp64_seed(er_ctx* ctx, double* max_rel_err);
 /* Self-test of the kernels' bounded waits: one CTA waits, `spins` polls at
  * most, for a completion barrier that nothing completes; the wait must give
  * up, raise the context's fault word and let the host see it (ER_OK then;
- * ER_ERR_CUDA if it did not report). The context stays usable. The staged
- * producer (build option ER_BULK=1) waits the same way with 2^22 polls. No
- * counterpart in the reference. */
+ * ER_ERR_CUDA if it did not report). The context stays usable. No counterpart
+ * in the reference. */
 int er_selftest_wait_timeout(er_ctx* ctx, int spins);
 
 /* Library version string. */

@@ -146,11 +146,12 @@ constexpr int grid_min_blocks() {
     return PREC == PREC_FP64 ? 2 : 3;
 }
 
-template <int PREC, int P>
+template <int PREC, int P, int SPLIT>
 __global__ void __launch_bounds__(kThreads, grid_min_blocks<PREC>())
     grid_kernel(const __grid_constant__ GridTask task) {
-    GridPolicy<P> pol(&task, blockIdx.x);
-    process_cta<GridPolicy<P>, PREC>(pol, task.fw, task.cc);
+    using Pol = GridPolicy<P, SPLIT>;
+    Pol pol(&task, blockIdx.x);
+    process_cta<Pol, PREC>(pol, task.fw, task.cc);
 }
 
 // A batch in one launch: CTA b is brick b - start[k] of task k, start[k] <= b <
@@ -199,25 +200,25 @@ __global__ void f32_to_f64_kernel(const float* __restrict__ in, double* __restri
         out[i] = (double)in[i];
 }
 
-template <int P>
+template <int P, int SPLIT>
 static int configure_variant(er_ctx* ctx) {
     const int smem = (int)sizeof(EngineSmem);
-    ER_CUDA(ctx, cudaFuncSetAttribute(grid_kernel<PREC_COMP, P>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ER_CUDA(ctx, cudaFuncSetAttribute(grid_kernel<PREC_FP32, P>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ER_CUDA(ctx, cudaFuncSetAttribute(grid_kernel<PREC_COUNT, P>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ER_CUDA(ctx, cudaFuncSetAttribute(grid_kernel<PREC_NEAR64, P>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ER_CUDA(ctx, cudaFuncSetAttribute(grid_kernel<PREC_FP64, P>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    const auto set = [&](auto* kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    };
+    ER_CUDA(ctx, set(grid_kernel<PREC_COMP, P, SPLIT>));
+    ER_CUDA(ctx, set(grid_kernel<PREC_FP32, P, SPLIT>));
+    ER_CUDA(ctx, set(grid_kernel<PREC_COUNT, P, SPLIT>));
+    ER_CUDA(ctx, set(grid_kernel<PREC_NEAR64, P, SPLIT>));
+    ER_CUDA(ctx, set(grid_kernel<PREC_FP64, P, SPLIT>));
     return ER_OK;
 }
 
 static int configure_kernels(er_ctx* ctx) {
-    int st = configure_variant<4>(ctx);
-    if (st == ER_OK) st = configure_variant<8>(ctx);
+    int st = configure_variant<4, 1>(ctx);
+    if (st == ER_OK) st = configure_variant<8, 1>(ctx);
+    if (st == ER_OK) st = configure_variant<4, 2>(ctx);
+    if (st == ER_OK) st = configure_variant<4, 4>(ctx);
     const int smem = (int)sizeof(EngineSmem);
     ER_CUDA(ctx, cudaFuncSetAttribute(grid_batch_kernel<PREC_COMP>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -254,24 +255,34 @@ int fill_grid_task(er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, floa
 
 static int64_t task_bricks(const GridTask& t) { return (int64_t)t.nb[0] * t.nb[1] * t.nb[2]; }
 
+// CTAs per brick of a P = 4 grid: 4 while they have an SM each, 2 while they
+// fit the three slots an SM has, 1 from there on (a second wave of split CTAs
+// costs more than the idle slots). Same bits in every case. Measured unsplit /
+// 2 / 4, us a call, 424-atom cell: 16^3 136 / 77 / 66, 32^3 (32 bricks) 55 / 41
+// / 37, 40^3 (75) 51 / 43 / 53, 56^3 (196) 59 / 54 / 76, 64^3 (256) 56 / 68 / 95.
+static int grid_split(const er_ctx* ctx, int64_t bricks) {
+    if (4 * bricks <= ctx->num_sms) return 4;
+    return 2 * bricks <= 3 * ctx->num_sms ? 2 : 1;
+}
+
+template <int P, int SPLIT>
+static void launch_variant(const GridTask& t, int prec, unsigned bricks, cudaStream_t st) {
+    const size_t smem = sizeof(EngineSmem);
+    const unsigned g = bricks * SPLIT;
+    if (prec == PREC_FP32) grid_kernel<PREC_FP32, P, SPLIT><<<g, kThreads, smem, st>>>(t);
+    else if (prec == PREC_COUNT) grid_kernel<PREC_COUNT, P, SPLIT><<<g, kThreads, smem, st>>>(t);
+    else if (prec == PREC_NEAR64) grid_kernel<PREC_NEAR64, P, SPLIT><<<g, kThreads, smem, st>>>(t);
+    else if (prec == PREC_FP64) grid_kernel<PREC_FP64, P, SPLIT><<<g, kThreads, smem, st>>>(t);
+    else grid_kernel<PREC_COMP, P, SPLIT><<<g, kThreads, smem, st>>>(t);
+}
+
 int launch_grid_plain_on(er_ctx* ctx, const GridTask& t, int prec, cudaStream_t st) {
     const int64_t nbr = task_bricks(t);
     if (nbr > INT32_MAX) return set_error(ctx, ER_ERR_LIMIT, "grid: too many bricks");
-    const size_t smem = sizeof(EngineSmem);
-    const unsigned g = (unsigned)nbr;
-    if (t.tile_p == 8) {
-        if (prec == PREC_FP32) grid_kernel<PREC_FP32, 8><<<g, kThreads, smem, st>>>(t);
-        else if (prec == PREC_COUNT) grid_kernel<PREC_COUNT, 8><<<g, kThreads, smem, st>>>(t);
-        else if (prec == PREC_NEAR64) grid_kernel<PREC_NEAR64, 8><<<g, kThreads, smem, st>>>(t);
-        else if (prec == PREC_FP64) grid_kernel<PREC_FP64, 8><<<g, kThreads, smem, st>>>(t);
-        else grid_kernel<PREC_COMP, 8><<<g, kThreads, smem, st>>>(t);
-    } else {
-        if (prec == PREC_FP32) grid_kernel<PREC_FP32, 4><<<g, kThreads, smem, st>>>(t);
-        else if (prec == PREC_COUNT) grid_kernel<PREC_COUNT, 4><<<g, kThreads, smem, st>>>(t);
-        else if (prec == PREC_NEAR64) grid_kernel<PREC_NEAR64, 4><<<g, kThreads, smem, st>>>(t);
-        else if (prec == PREC_FP64) grid_kernel<PREC_FP64, 4><<<g, kThreads, smem, st>>>(t);
-        else grid_kernel<PREC_COMP, 4><<<g, kThreads, smem, st>>>(t);
-    }
+    if (t.tile_p == 8) launch_variant<8, 1>(t, prec, (unsigned)nbr, st);
+    else if (grid_split(ctx, nbr) == 4) launch_variant<4, 4>(t, prec, (unsigned)nbr, st);
+    else if (grid_split(ctx, nbr) == 2) launch_variant<4, 2>(t, prec, (unsigned)nbr, st);
+    else launch_variant<4, 1>(t, prec, (unsigned)nbr, st);
     ER_CUDA(ctx, cudaGetLastError());
     return ER_OK;
 }

@@ -341,24 +341,47 @@ __device__ __forceinline__ float pair_term(float r2, float c12, float nc6) {
 // lattice lines are its values at corners of the set, bit for bit. With every
 // point forming its own divisions twice and FP64 shuffles for the boxes, this
 // took 11,000 of the 84,000 clocks of a CTA (129^3 grid of a 424-atom cell).
-template <int P_>
-struct GridPolicy {
-    static constexpr int kP = P_;
+//
+// SPLIT > 1 spreads one brick over SPLIT CTAs, for grids of few bricks: CTA
+// `item % SPLIT` takes kWarps / SPLIT of the sub-bricks, SPLIT warps to each
+// with P / SPLIT of its points a lane. Box, origin, candidates and lists stay
+// those of the brick and the sub-brick, so every energy keeps its bits.
+template <int SPLIT>
+struct BrickPart {  // which of its brick's SPLIT CTAs this is
+    int part;
+    __device__ explicit BrickPart(int item) : part(item % SPLIT) {}
+};
+template <>
+struct BrickPart<1> {
+    static constexpr int part = 0;
+    __device__ explicit BrickPart(int) {}
+};
+
+template <int P_, int SPLIT = 1>
+struct GridPolicy : BrickPart<SPLIT> {
+    static constexpr int kP = P_ / SPLIT, kBoxP = kP;
     static constexpr bool kLattice = true;
     static constexpr int kBI = 2 * P_, kBJ = 2 * kWJ, kBK = 2 * kWK;
+    static_assert(P_ % SPLIT == 0 && kWarps % SPLIT == 0, "whole points and sub-bricks per warp");
     const GridTask* T;
     int i0, j0, k0;
-    __device__ GridPolicy(const GridTask* task, int brick) : T(task) {
+    __device__ GridPolicy(const GridTask* task, int item) : BrickPart<SPLIT>(item), T(task) {
+        const int brick = item / SPLIT;
         const int nbk = task->nb[2], nbj = task->nb[1];
         const int bk = brick % nbk;
         const int bj = (brick / nbk) % nbj;
         const int bi = brick / (nbk * nbj);
         i0 = bi * kBI; j0 = bj * kBJ; k0 = bk * kBK;
     }
+    // the sub-brick of warp w
+    __device__ __forceinline__ int sub(int w) const {
+        return this->part * (kWarps / SPLIT) + w / SPLIT;
+    }
     __device__ __forceinline__ void index(int w, int lane, int p, int& i, int& j, int& k) const {
-        i = i0 + (w & 1) * kP + p;
-        j = j0 + ((w >> 1) & 1) * kWJ + lane / kWK;
-        k = k0 + (w >> 2) * kWK + lane % kWK;
+        const int b = sub(w);
+        i = i0 + (b & 1) * P_ + w % SPLIT * kP + p;
+        j = j0 + ((b >> 1) & 1) * kWJ + lane / kWK;
+        k = k0 + (b >> 2) * kWK + lane % kWK;
     }
     // One thread per lattice line; the caller synchronises. Lines past the
     // grid repeat its last one (such points are never stored).
@@ -421,7 +444,8 @@ struct GridPolicy {
     }
     __device__ __forceinline__ bool warp_box(const double* r, int w, double* lo,
                                              double* hi) const {
-        return box(r, (w & 1) * kP, kP, ((w >> 1) & 1) * kWJ, kWJ, (w >> 2) * kWK, kWK, lo, hi);
+        const int b = sub(w);
+        return box(r, (b & 1) * P_, P_, ((b >> 1) & 1) * kWJ, kWJ, (b >> 2) * kWK, kWK, lo, hi);
     }
     __device__ __forceinline__ void store(int w, int lane, int p, float e) const {
         int i, j, k;
@@ -441,33 +465,60 @@ struct GridPolicy {
 
 // Widom insertion points: CTA c owns sorted positions [256 P c, 256 P (c + 1))
 // of `order` (points stored in that order); warp w the 32 P positions from
-// 256 P c + 32 P w, lane l position p * 32 + l of them.
-template <int P_>
-struct PointPolicy {
-    static constexpr int kP = P_;
+// 256 P c + 32 P w, lane l position p * 32 + l of them. SPLIT > 1 as for grid
+// bricks: SPLIT CTAs share those positions, SPLIT warps a warp's 32 P of them.
+template <int P_, int SPLIT = 1>
+struct PointPolicy : BrickPart<SPLIT> {
+    static constexpr int kP = P_ / SPLIT;
+    static constexpr int kBoxP = P_;  // points per lane of the box passes
     static constexpr bool kLattice = false;
+    static_assert(P_ % SPLIT == 0 && kWarps % SPLIT == 0, "whole points and warps");
     const PointTask* T;
     int base, nv;
-    __device__ PointPolicy(const PointTask* task, int cta)
-        : T(task), base(cta * kWarps * 32 * kP), nv(*task->n_valid) {}
+    __device__ PointPolicy(const PointTask* task, int item)
+        : BrickPart<SPLIT>(item), T(task), base(item / SPLIT * (kWarps * 32 * P_)),
+          nv(*task->n_valid) {}
+    // the position of point p of lane `lane`, warp w
+    __device__ __forceinline__ int raw_pos(int w, int lane, int p) const {
+        return base + (this->part * (kWarps / SPLIT) + w / SPLIT) * (32 * P_) +
+               (w % SPLIT * kP + p) * 32 + lane;
+    }
     __device__ __forceinline__ int slot_index(int w, int lane, int p) const {
-        const int pos = base + w * (32 * kP) + p * 32 + lane;
+        const int pos = raw_pos(w, lane, p);
         return pos < nv ? T->order[pos] : -1;
     }
     __device__ __forceinline__ int pos_of(int w, int lane, int p, bool& ok) const {
-        const int pos = base + w * (32 * kP) + p * 32 + lane;
+        const int pos = raw_pos(w, lane, p);
         ok = pos < nv;
         return ok ? pos : min(base, nv - 1);  // a finite stand-in, never stored
+    }
+    // Cartesian position of a sorted position that is in range
+    __device__ __forceinline__ void at(int pos, double& x, double& y, double& z) const {
+        x = T->pts[3 * (size_t)pos];
+        y = T->pts[3 * (size_t)pos + 1];
+        z = T->pts[3 * (size_t)pos + 2];
+    }
+    // point q (of kBoxP) that warp w brings to the CTA box, and to the box of
+    // the 32 P positions it works on
+    __device__ __forceinline__ bool cta_point(int w, int lane, int q, double& x, double& y,
+                                              double& z) const {
+        const int pos = base + w * (32 * P_) + q * 32 + lane;
+        if (pos < nv) at(pos, x, y, z);
+        return pos < nv;
+    }
+    __device__ __forceinline__ bool warp_point(int w, int lane, int q, double& x, double& y,
+                                               double& z) const {
+        const int pos =
+            base + (this->part * (kWarps / SPLIT) + w / SPLIT) * (32 * P_) + q * 32 + lane;
+        if (pos < nv) at(pos, x, y, z);
+        return pos < nv;
     }
     // Cartesian position (frame r), stored at its bin-order position by the
     // placement pass
     __device__ __forceinline__ bool cart(const double*, int w, int lane, int p, double& x,
                                          double& y, double& z) const {
         bool ok;
-        const int pos = pos_of(w, lane, p, ok);
-        x = T->pts[3 * (size_t)pos];
-        y = T->pts[3 * (size_t)pos + 1];
-        z = T->pts[3 * (size_t)pos + 2];
+        at(pos_of(w, lane, p, ok), x, y, z);
         return ok;
     }
     // fractional position, regenerated from the insertion's Philox counter
@@ -852,87 +903,96 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
     return nrec;
 }
 
-// Generic (per-point x, y, z) inner and shell lists, scalar FP32.
+// Inner and shell lists of a lane's one point (split bricks), kBatch atoms at a
+// time. Per point the same operations in the same order as the packed forms
+// above, so the energies are theirs bit for bit.
 template <class Pol, int PREC>
-__device__ __forceinline__ int generic_lists(EngineSmem& s, const unsigned short* wl,
-                                             int n_in, int n_sh, float rc2f, float win,
-                                             Lane<Pol, PREC>& L, unsigned& rec) {
-    constexpr int P = Pol::kP;
+__device__ __forceinline__ int single_lists(EngineSmem& s, const unsigned short* wl, int n_in,
+                                            int n_sh, float rc2f, float win,
+                                            Lane<Pol, PREC>& L, unsigned& rec) {
     constexpr bool kComp = PrecTraits<PREC>::comp;
-    float acc[P];
+    constexpr int kBatch = 4;
+    const float px = L.px[0], py = L.py[0], pz = L.pz[0];
+    const char* cbase = reinterpret_cast<const char*>(s.cand);
+    float acc = 0.f;
+    auto r2_of = [&](const float4 v) {  // x x y z
+        return Pol::kLattice ? r2_lattice(px, v.x, ss_lattice(py, pz, v.z, v.w))
+                             : r2_generic(px, py, pz, v.x, v.z, v.w);
+    };
+    auto load = [&](unsigned off, float4& v0, float4& v1) {
+        v0 = *reinterpret_cast<const float4*>(cbase + off);
+        v1 = *reinterpret_cast<const float4*>(cbase + off + 16);
+    };
+    auto inner = [&](auto n_, const unsigned short* l) {
+        constexpr int N = decltype(n_)::value;
+        float4 v0[N], v1[N];
 #pragma unroll
-    for (int p = 0; p < P; ++p) acc[p] = 0.f;
+        for (int k = 0; k < N; ++k) load(l[k], v0[k], v1[k]);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (PREC == PREC_COUNT) {
+                acc += 1.0f;
+            } else {
+                const float u = rcp_approx(r2_of(v0[k]));
+                const float u3 = __fmul_rn(__fmul_rn(u, u), u);
+                acc = __fmaf_rn(u3, __fmaf_rn(v1[k].x, u3, v1[k].z), acc);
+            }
+        }
+    };
+    double acc64 = 0.0;
     int q = 0;
     while (q < n_in) {
         const int qe = kComp ? min(q + PrecTraits<PREC>::inner_chunk, n_in) : n_in;
-#pragma unroll 2
-        for (; q < qe; ++q) {
-            const Cand& cd = *reinterpret_cast<const Cand*>(
-                reinterpret_cast<const char*>(s.cand) + wl[q]);
-            const float4 v0 = *reinterpret_cast<const float4*>(&cd.ax);   // x - y z
-            const float4 v1 = *reinterpret_cast<const float4*>(&cd.c12);  // C12 - -C6 -
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                if (PREC == PREC_COUNT) {
-                    acc[p] += 1.0f;
-                } else {
-                    const float r2 = r2_generic(L.px[p], L.py[p], L.pz[p], v0.x, v0.z, v0.w);
-                    const float u = rcp_approx(r2);
-                    const float u3 = __fmul_rn(__fmul_rn(u, u), u);
-                    acc[p] = __fmaf_rn(u3, __fmaf_rn(v1.x, u3, v1.z), acc[p]);
-                }
-            }
-        }
-        if (kComp) {
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                tot_at(s, p) += (double)acc[p];
-                acc[p] = 0.f;
-            }
+        for (; q + kBatch <= qe; q += kBatch) inner(Int<kBatch>{}, wl + q);
+        for (; q < qe; ++q) inner(Int<1>{}, wl + q);
+        if (kComp || Pol::kLattice) {
+            acc64 += (double)acc;
+            acc = 0.f;
         }
     }
+    if (kComp || Pol::kLattice) tot_at(s, 0) += acc64;
     int nrec = 0;
     rec = 0;
+    auto shell = [&](auto n_, int q) {
+        constexpr int N = decltype(n_)::value;
+        float4 v0[N], v1[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) load(wl[kMaxCand - 1 - q - k], v0[k], v1[k]);
+        float d[N], all = INFINITY;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const float r2 = r2_of(v0[k]);
+            const float in = set_lt(r2, rc2f);
+            d[k] = fabsf(__fsub_rn(r2, rc2f));
+            all = fminf(all, d[k]);
+            if (PREC == PREC_COUNT) {
+                acc += in;
+            } else {
+                const float u = rcp_approx(r2);
+                const float u3 = __fmul_rn(__fmul_rn(u, u), u);
+                acc = __fmaf_rn(__fmul_rn(u3, in), __fmaf_rn(v1[k].x, u3, v1[k].z), acc);
+            }
+        }
+        if (all <= win) {  // rare: a pair of these atoms sits near the cutoff
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (d[k] <= win) {
+                    rec = (rec << 10) | (unsigned)(q + k);
+                    ++nrec;
+                }
+        }
+    };
     q = 0;
     while (q < n_sh) {
         const int qe = kComp ? min(q + kAccChunk, n_sh) : n_sh;
-#pragma unroll 2
-        for (; q < qe; ++q) {
-            const Cand& cd = *reinterpret_cast<const Cand*>(
-                reinterpret_cast<const char*>(s.cand) + wl[kMaxCand - 1 - q]);
-            const float4 v0 = *reinterpret_cast<const float4*>(&cd.ax);   // x - y z
-            const float4 v1 = *reinterpret_cast<const float4*>(&cd.c12);  // C12 - -C6 -
-            float mn = INFINITY;
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                const float r2 = r2_generic(L.px[p], L.py[p], L.pz[p], v0.x, v0.z, v0.w);
-                const float dd = __fsub_rn(r2, rc2f);
-                if (PREC == PREC_COUNT) {
-                    if (dd < 0.f) acc[p] += 1.0f;
-                } else {
-                    const float u = rcp_approx(r2);
-                    const float u3 = __fmul_rn(__fmul_rn(u, u), u);
-                    if (dd < 0.f) acc[p] = __fmaf_rn(u3, __fmaf_rn(v1.x, u3, v1.z), acc[p]);
-                }
-                mn = fminf(mn, fabsf(dd));
-            }
-            if (mn <= win) {  // rare: a pair of this atom sits near the cutoff
-                rec = (rec << 10) | (unsigned)q;
-                ++nrec;
-            }
-        }
+        for (; q + kBatch <= qe; q += kBatch) shell(Int<kBatch>{}, q);
+        for (; q < qe; ++q) shell(Int<1>{}, q);
         if (kComp) {
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                tot_at(s, p) += (double)acc[p];
-                acc[p] = 0.f;
-            }
+            tot_at(s, 0) += (double)acc;
+            acc = 0.f;
         }
     }
-    if (!kComp) {
-#pragma unroll
-        for (int p = 0; p < P; ++p) tot_at(s, p) += (double)acc[p];
-    }
+    if (!kComp) tot_at(s, 0) += (double)acc;
     return nrec;
 }
 
@@ -1225,13 +1285,13 @@ __device__ __forceinline__ void warp_flush(EngineSmem& s, const Pol& pol, const 
         return;
     }
 
-    if (Pol::kLattice) {
+    if constexpr (P == 1) {
+        nrec = single_lists<Pol, PREC>(s, wl, n_in, n_sh, rc2f, win, L, rec);
+    } else if constexpr (Pol::kLattice) {
         lattice_inner<Pol, PREC>(s, wl, n_in, L);
         nrec = lattice_shell<Pol, PREC>(s, wl, n_sh, rc2f, win, L, rec);
     } else {
-        nrec = (Pol::kP % 2 == 0)
-                   ? generic_packed_lists<Pol, PREC>(s, wl, n_in, n_sh, rc2f, win, L, rec)
-                   : generic_lists<Pol, PREC>(s, wl, n_in, n_sh, rc2f, win, L, rec);
+        nrec = generic_packed_lists<Pol, PREC>(s, wl, n_in, n_sh, rc2f, win, L, rec);
     }
 
     // --- exact re-decision of borderline shell pairs (rare); lanes without a
@@ -1262,9 +1322,12 @@ __device__ void process_cta(const Pol& pol, const FwDev& fw, const CutoffConsts&
         double mn0 = INFINITY, mn1 = INFINITY, mn2 = INFINITY;
         double mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY;
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
+        for (int q = 0; q < Pol::kBoxP; ++q) {
             double x, y, z;
-            if (pol.cart(fw.r, w, lane, p, x, y, z)) {
+            // (unsplit, the CTA's points are its own lanes')
+            const bool ok = Pol::kBoxP == P ? pol.cart(fw.r, w, lane, q, x, y, z)
+                                            : pol.cta_point(w, lane, q, x, y, z);
+            if (ok) {
                 mn0 = fmin(mn0, x); mn1 = fmin(mn1, y); mn2 = fmin(mn2, z);
                 mx0 = fmax(mx0, x); mx1 = fmax(mx1, y); mx2 = fmax(mx2, z);
             }
@@ -1316,7 +1379,8 @@ __device__ void process_cta(const Pol& pol, const FwDev& fw, const CutoffConsts&
                 L.pz[Pol::kLattice ? 0 : p] = fz;
             }
             tot_at(s, p) = 0.0;
-            if (!Pol::kLattice && (L.vmask & (1u << p))) {
+            // (unsplit, the warp's points are its own lanes')
+            if (!Pol::kLattice && Pol::kBoxP == P && (L.vmask & (1u << p))) {
                 wl0x = fminf(wl0x, fx); wl0y = fminf(wl0y, fy); wl0z = fminf(wl0z, fz);
                 wh0x = fmaxf(wh0x, fx); wh0y = fmaxf(wh0y, fy); wh0z = fmaxf(wh0z, fz);
             }
@@ -1330,6 +1394,15 @@ __device__ void process_cta(const Pol& pol, const FwDev& fw, const CutoffConsts&
                 wh0x = (float)(hi[0] - o0); wh0y = (float)(hi[1] - o1); wh0z = (float)(hi[2] - o2);
             }
         } else {
+#pragma unroll
+            for (int q = 0; q < (Pol::kBoxP == P ? 0 : Pol::kBoxP); ++q) {
+                double x, y, z;
+                if (pol.warp_point(w, lane, q, x, y, z)) {
+                    const float fx = (float)(x - o0), fy = (float)(y - o1), fz = (float)(z - o2);
+                    wl0x = fminf(wl0x, fx); wl0y = fminf(wl0y, fy); wl0z = fminf(wl0z, fz);
+                    wh0x = fmaxf(wh0x, fx); wh0y = fmaxf(wh0y, fy); wh0z = fmaxf(wh0z, fz);
+                }
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 wl0x = fminf(wl0x, __shfl_xor_sync(0xffffffffu, wl0x, o));

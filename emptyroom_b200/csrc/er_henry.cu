@@ -374,14 +374,15 @@ __global__ void henry_order_straddling_kernel(const int* __restrict__ starts, in
     }
 }
 
-template <int P>
+template <int P, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 2)
     henry_energy_kernel(const __grid_constant__ PointTask task) {
-    if ((long long)blockIdx.x * (kWarps * 32 * P) >= (long long)*task.n_valid) return;
-    PointPolicy<P> pol(&task, blockIdx.x);
+    if ((long long)(blockIdx.x / SPLIT) * (kWarps * 32 * P) >= (long long)*task.n_valid) return;
+    using Pol = PointPolicy<P, SPLIT>;
+    Pol pol(&task, blockIdx.x);
     // near pairs in FP64: a Boltzmann factor turns an energy error dE into a
     // relative weight error dE / T, so Widom energies get the tighter mode
-    process_cta<PointPolicy<P>, PREC_NEAR64>(pol, task.fw, task.cc);
+    process_cta<Pol, PREC_NEAR64>(pol, task.fw, task.cc);
 }
 
 __device__ __forceinline__ Lse lse_merge(Lse a, Lse b) {
@@ -581,17 +582,23 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
     const int hp = henry_points_per_thread(n);
     const int per_cta = kWarps * 32 * hp;
     const int ecta = (n + per_cta - 1) / per_cta;
-    if (hp == kHenryP) {
-        ER_CUDA(ctx, cudaFuncSetAttribute(henry_energy_kernel<kHenryP>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)sizeof(EngineSmem)));
-        henry_energy_kernel<kHenryP><<<ecta, kThreads, sizeof(EngineSmem), st>>>(task);
-    } else {
-        ER_CUDA(ctx, cudaFuncSetAttribute(henry_energy_kernel<kHenryPSmall>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)sizeof(EngineSmem)));
-        henry_energy_kernel<kHenryPSmall><<<ecta, kThreads, sizeof(EngineSmem), st>>>(task);
-    }
+    auto energy = [&](auto* kernel, int split) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EngineSmem));
+        if (e == cudaSuccess) kernel<<<ecta * split, kThreads, sizeof(EngineSmem), st>>>(task);
+        return e;
+    };
+    // runs of few CTAs share each CTA's points among several (same bits): four
+    // while a CTA has an SM, two while the halves fit an SM's two slots.
+    // Measured whole / 2 / 4, us a call, 424-atom cell: 16k insertions 187 /
+    // 143 / 127, 32k 169 / 136 / 126, 65k 149 / 125 / 126, 100k 139 / 135 / 149,
+    // 150k 138 / 137 / 162, 400k 192 / 212 / 265.
+    if (hp == kHenryP) ER_CUDA(ctx, energy(henry_energy_kernel<kHenryP, 1>, 1));
+    else if (2 * ecta <= ctx->num_sms)
+        ER_CUDA(ctx, energy(henry_energy_kernel<kHenryPSmall, 4>, 4));
+    else if (ecta <= ctx->num_sms)
+        ER_CUDA(ctx, energy(henry_energy_kernel<kHenryPSmall, 2>, 2));
+    else ER_CUDA(ctx, energy(henry_energy_kernel<kHenryPSmall, 1>, 1));
     ER_CUDA(ctx, cudaGetLastError());
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[3], st));
     const int rblocks = std::min(4096, std::max(1, ctx->num_sms * 4));

@@ -202,15 +202,15 @@ __global__ void f32_to_f64_kernel(const float* __restrict__ in, double* __restri
 
 template <int P, int SPLIT>
 static int configure_variant(er_ctx* ctx) {
-    const int smem = (int)sizeof(EngineSmem);
-    const auto set = [&](auto* kernel) {
-        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const auto set = [&](auto* kernel, int prec) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)engine_smem_bytes(prec));
     };
-    ER_CUDA(ctx, set(grid_kernel<PREC_COMP, P, SPLIT>));
-    ER_CUDA(ctx, set(grid_kernel<PREC_FP32, P, SPLIT>));
-    ER_CUDA(ctx, set(grid_kernel<PREC_COUNT, P, SPLIT>));
-    ER_CUDA(ctx, set(grid_kernel<PREC_NEAR64, P, SPLIT>));
-    ER_CUDA(ctx, set(grid_kernel<PREC_FP64, P, SPLIT>));
+    ER_CUDA(ctx, set(grid_kernel<PREC_COMP, P, SPLIT>, PREC_COMP));
+    ER_CUDA(ctx, set(grid_kernel<PREC_FP32, P, SPLIT>, PREC_FP32));
+    ER_CUDA(ctx, set(grid_kernel<PREC_COUNT, P, SPLIT>, PREC_COUNT));
+    ER_CUDA(ctx, set(grid_kernel<PREC_NEAR64, P, SPLIT>, PREC_NEAR64));
+    ER_CUDA(ctx, set(grid_kernel<PREC_FP64, P, SPLIT>, PREC_FP64));
     return ER_OK;
 }
 
@@ -267,7 +267,7 @@ static int grid_split(const er_ctx* ctx, int64_t bricks) {
 
 template <int P, int SPLIT>
 static void launch_variant(const GridTask& t, int prec, unsigned bricks, cudaStream_t st) {
-    const size_t smem = sizeof(EngineSmem);
+    const size_t smem = engine_smem_bytes(prec);
     const unsigned g = bricks * SPLIT;
     if (prec == PREC_FP32) grid_kernel<PREC_FP32, P, SPLIT><<<g, kThreads, smem, st>>>(t);
     else if (prec == PREC_COUNT) grid_kernel<PREC_COUNT, P, SPLIT><<<g, kThreads, smem, st>>>(t);

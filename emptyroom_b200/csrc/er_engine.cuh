@@ -114,12 +114,31 @@ struct __align__(32) EngineSmem {
     double axis[kAxisMax];                 // fractional coordinates of a brick's lattice lines
 };
 
+// Atoms a warp holds in FP64 (near_lists, fp64_lists): position relative to the
+// CTA centre and FP64 (C12, C6).
+struct __align__(16) NearAtom {
+    double x, y, z, c12, c6, pad;
+};
+constexpr int kNearStage = 32;  // one per lane
+// Shared memory of a block: PREC_FP64 has a stage per warp behind EngineSmem
+// (its two CTAs per SM have the room), PREC_NEAR64 uses a consumed list.
+__host__ __device__ constexpr size_t engine_smem_bytes(int prec) {
+    return sizeof(EngineSmem) +
+           (prec == PREC_FP64 ? kWarps * kNearStage * sizeof(NearAtom) : (size_t)0);
+}
+
 // The block's EngineSmem, by the shared array itself: a reference handed to an
 // out-of-line function arrives as a generic pointer, and the pair loops then
 // run on generic loads (half again as long in a 32^3 grid).
 __device__ __forceinline__ EngineSmem& engine_smem() {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     return *reinterpret_cast<EngineSmem*>(smem_raw);
+}
+// This warp's stage of PREC_FP64.
+__device__ __forceinline__ NearAtom* fp64_stage() {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    return reinterpret_cast<NearAtom*>(smem_raw + sizeof(EngineSmem)) +
+           (threadIdx.x >> 5) * kNearStage;
 }
 
 // ----------------------------------------------------------- packed FP32x2
@@ -253,18 +272,6 @@ __device__ __forceinline__ Atom64 atom64(const FwDev& fw, int gid, double o0, do
     const double4 a = fw.img_xyz[gid];
     const double2 lj = fw.img_lj64[gid];
     return Atom64{a.x - o0, a.y - o1, a.z - o2, lj.x, lj.y};
-}
-// FP64 pair term of atom a at a point q (both relative to the CTA centre),
-// with the correctly rounded reciprocal (ER_PREC_FP64, the reference mode of
-// the precision sweeps).
-__device__ __forceinline__ double pair64(const Atom64& a, double qx, double qy, double qz,
-                                         double r2min) {
-    const double dx = qx - a.x, dy = qy - a.y, dz = qz - a.z;
-    double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-    r2 = fmax(r2, r2min);
-    const double u = __drcp_rn(r2);
-    const double u3 = u * u * u;
-    return u3 * fma(a.c12, u3, -a.c6);
 }
 // 1/x in FP64 for the near pairs of PREC_NEAR64: one Newton step
 // y = y0 (1 + e), e = 1 - x y0, from the hardware seed y0 =
@@ -1052,10 +1059,6 @@ static __device__ __noinline__ void recheck_borderline(const Pol& pol, const FwD
 // dependent load -- is paid once per 32 atoms instead of once per atom, and
 // every lane reads the atoms back by broadcast. Out of line: its FP64 state
 // stays out of the FP32 loops' registers.
-struct __align__(16) NearAtom {
-    double x, y, z, c12, c6, pad;
-};
-constexpr int kNearStage = 32;
 static_assert(kNearStage * sizeof(NearAtom) <= kMaxCand * sizeof(unsigned short),
               "the staged atoms fit a warp's list");
 
@@ -1164,6 +1167,89 @@ static __device__ __noinline__ void near_lists(const Pol& pol, const FwDev& fw,
     }
 }
 
+// Inner and shell lists of PREC_FP64: every pair term in FP64 (the reference
+// mode of the precision sweeps, and a caller's choice), shell pairs decided on
+// their FP32 r^2 and by exact_in_cutoff inside the error window. Atoms are
+// fetched 32 at a time as in near_lists and serve all of a lane's points; with
+// every point fetching every atom the 65 x 63 x 61 grid of a 424-atom cell took
+// 280 us, now 167 (bound by FP64 arithmetic, 22 operations a pair).
+template <class Pol, int PREC>
+__device__ __forceinline__ void fp64_lists(EngineSmem& s, const Pol& pol, const FwDev& fw,
+                                           const CutoffConsts& cc, const unsigned short* wl,
+                                           int n_in, int n_sh, float win,
+                                           const Lane<Pol, PREC>& L) {
+    constexpr int P = Pol::kP;
+    static_assert(Pol::kLattice, "grids only");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    NearAtom* st = fp64_stage();
+    double qx[P], qy, qz, acc[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        pol.cart(fw.r, w, lane, p, qx[p], qy, qz);
+        qx[p] -= s.org[0];
+        acc[p] = 0.0;
+    }
+    qy -= s.org[1];
+    qz -= s.org[2];
+    // list entries q0 .. of a list of n: `step` = 1 from its front, -1 from its back
+    auto stage = [&](const unsigned short* list, int step, int q0, int n) {
+        __syncwarp();
+        if (q0 + lane < n) {
+            const Atom64 a = atom64(fw, s.cid[list[step * (q0 + lane)] >> 5], s.org[0], s.org[1],
+                                    s.org[2]);
+            NearAtom& d = st[lane];
+            *reinterpret_cast<double2*>(&d.x) = make_double2(a.x, a.y);
+            *reinterpret_cast<double2*>(&d.z) = make_double2(a.z, a.c12);
+            d.c6 = a.c6;
+        }
+        __syncwarp();
+    };
+    // the correctly rounded reciprocal: a seed refined twice took 31 us less
+    // and left errors up to 9 % larger (against 64-bit sums, eight grids)
+    auto term = [&](const NearAtom& a, double dy, double dz, int p) {
+        const double dx = qx[p] - a.x;
+        const double u = __drcp_rn(fmax(fma(dz, dz, fma(dy, dy, dx * dx)), cc.r2min));
+        const double u3 = u * u * u;
+        return u3 * fma(a.c12, u3, -a.c6);
+    };
+    for (int q0 = 0; q0 < n_in; q0 += kNearStage) {
+        stage(wl, 1, q0, n_in);
+        const int m = min(kNearStage, n_in - q0);
+        for (int k = 0; k < m; ++k) {
+            const NearAtom a = st[k];
+            const double dy = qy - a.y, dz = qz - a.z;
+#pragma unroll
+            for (int p = 0; p < P; ++p) acc[p] += term(a, dy, dz, p);
+        }
+    }
+    const unsigned short* back = wl + kMaxCand - 1;
+    for (int q0 = 0; q0 < n_sh; q0 += kNearStage) {
+        stage(back, -1, q0, n_sh);
+        const int m = min(kNearStage, n_sh - q0);
+        for (int k = 0; k < m; ++k) {
+            const NearAtom a = st[k];
+            const unsigned off = back[-(q0 + k)];
+            const Cand& cd = s.cand[off >> 5];
+            const float ss = ss_lattice(L.py[0], L.pz[0], cd.ay, cd.az);
+            const double dy = qy - a.y, dz = qz - a.z;
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                const float dd = __fsub_rn(r2_lattice(L.px[p], cd.ax, ss), cc.rc2f);
+                bool inside = dd < 0.f;
+                if (fabsf(dd) <= win) {
+                    double f[3];
+                    pol.point(w, lane, p, f);
+                    inside = exact_in_cutoff(fw, f, s.cid[off >> 5], cc.r2min);
+                }
+                const double e = term(a, dy, dz, p);
+                if (inside) acc[p] += e;
+            }
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) tot_at(s, p) += acc[p];
+}
+
 template <class Pol, int PREC>
 __device__ __forceinline__ void warp_flush(EngineSmem& s, const Pol& pol, const FwDev& fw,
                                                 const CutoffConsts& cc, int n_cand,
@@ -1239,49 +1325,10 @@ __device__ __forceinline__ void warp_flush(EngineSmem& s, const Pol& pol, const 
         win = ldexpf((float)L.bul, e - 24);
     }
 
-    // FP64 positions of this lane's points relative to the CTA centre
-    // (FP64 paths only).
-    auto point64 = [&](int p, double& qx, double& qy, double& qz) {
-        double x, y, z, o0, o1, o2;
-        pol.cart(fw.r, w, lane, p, x, y, z);
-        cta_centre(s, o0, o1, o2);
-        qx = x - o0;
-        qy = y - o1;
-        qz = z - o2;
-    };
-
     int nrec = 0;
     unsigned rec = 0;
-    if (kF64) {
-        // every inner pair in FP64; shell pairs decided as below, term in FP64
-        double o0, o1, o2;
-        cta_centre(s, o0, o1, o2);
-#pragma unroll 1
-        for (int p = 0; p < P; ++p) {
-            double qx, qy, qz;
-            point64(p, qx, qy, qz);
-            double acc = 0.0;
-            for (int q = 0; q < n_in; ++q)
-                acc += pair64(atom64(fw, s.cid[wl[q] >> 5], o0, o1, o2), qx, qy, qz, cc.r2min);
-            double f[3];
-            pol.point(w, lane, p, f);
-            for (int q = 0; q < n_sh; ++q) {
-                const unsigned off = wl[kMaxCand - 1 - q];
-                const Cand& cd = s.cand[off >> 5];
-                const float r2 = Pol::kLattice
-                                     ? r2_lattice(L.px[p], cd.ax, ss_lattice(L.py[0], L.pz[0],
-                                                                             cd.ay, cd.az))
-                                     : r2_generic(L.px[p], L.py[Pol::kLattice ? 0 : p],
-                                                  L.pz[Pol::kLattice ? 0 : p], cd.ax, cd.ay,
-                                                  cd.az);
-                const float dd = __fsub_rn(r2, rc2f);
-                bool inside = dd < 0.f;
-                if (fabsf(dd) <= win) inside = exact_in_cutoff(fw, f, s.cid[off >> 5], cc.r2min);
-                if (inside)
-                    acc += pair64(atom64(fw, s.cid[off >> 5], o0, o1, o2), qx, qy, qz, cc.r2min);
-            }
-            tot_at(s, p) += acc;
-        }
+    if constexpr (kF64) {
+        fp64_lists<Pol, PREC>(s, pol, fw, cc, wl, n_in, n_sh, win, L);
         return;
     }
 

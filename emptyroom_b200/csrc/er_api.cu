@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, grid_min_blocks<PREC>())
 // (4 or 8 points per thread). The block scheduler hands the CTAs out in order
 // as SM slots fall free, which is the work queue: resident CTAs that pulled
 // items from a counter kept their loop's state in registers through the pair
-// loops and ran slower (8 triclinic frameworks, 84 M points: 17.36 against
+// loops and ran slower (8 triclinic frameworks, 54 M points: 17.36 against
 // 16.73 ms; 64 grids of 32^3 680 against 633 us a call).
 // With task_left given, the CTA that finishes a task's last brick raises the
 // task's flag in host-mapped memory (done_host), so the host can copy that
@@ -236,6 +236,56 @@ int check_grid_dims(er_ctx* ctx, int nx, int ny, int nz, const char* who) {
     return ER_OK;
 }
 
+// Squared distance from which on a P = 8 brick's atoms are interpolated (0: no
+// atom is). h = the larger spacing of the two interpolated axes. 46 h bounds the
+// interpolation error of the smooth attraction; 4 A + 16 h that of the steep
+// terms near 5 A, where 46 h alone is not far enough (h < 0.13 A: 2.7e-5 K root
+// mean square at 5.0 A and h = 0.1 A, 3e-6 K at 5.6 A); the near pairs' 5 A stay
+// outside. Grids coarser than about 0.2 A have no atom that far from a brick and
+// inside the cutoff of all its points.
+static float far_distance2(const FwRecord& fw, const GridTask& t, double* diag = nullptr) {
+    if (t.tile_p != 8) return 0.f;
+    const double ha = fw.cell_len[0] / (t.nx - 1), hc = fw.cell_len[2] / (t.nz - 1);
+    const double hm = std::max(ha, hc);
+    const double rf = std::max({(double)kNearR, 4.0 + 16.0 * hm, 46.0 * hm});
+    const double* r = fw.dev.r;
+    double diag2 = 0.0;  // of the brick's Cartesian box
+    for (int d = 0; d < 3; ++d) {
+        const double e = 15.0 * fabs(r[3 * d]) / (t.nx - 1) + 7.0 * fabs(r[3 * d + 1]) / (t.ny - 1) +
+                         15.0 * fabs(r[3 * d + 2]) / (t.nz - 1);
+        diag2 += e * e;
+    }
+    if (diag) *diag = sqrt(diag2);
+    return rf + sqrt(diag2) < sqrt(fw.rc2) ? (float)(rf * rf) : 0.f;
+}
+
+// P = 8 where its bricks have a far field of 32 atoms or more (the nodes and
+// barriers of a smaller one cost what it saves) and are enough to fill the GPU:
+// half its CTA slots while the spacing is fine, all of them where the far field
+// is small. Measured P = 4 / 8, us a call: 8 A cell at 0.1 A (250 bricks) 235 / 174,
+// 10 A at 0.13 A (250) 243 / 233, 14 A at 0.18 A (250) 265 / 286; 25.8 A cell of
+// 424 atoms at 0.17 A (1900) 385 / 375, at 0.15 A 553 / 474; of 2500 atoms at 0.17
+// A 2019 / 1897, at 0.13 A 4231 / 3093; of 150 atoms at 0.17 A (18 far atoms) 186
+// / 198, at 0.15 A (29) 266 / 266, at 0.12 A (41) 523 / 497.
+int default_tile(const er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, int prec) {
+    if (prec != PREC_NEAR64) return 4;
+    GridTask t;
+    t.tile_p = 8;
+    t.nx = nx; t.ny = ny; t.nz = nz;
+    double diag = 0.0;
+    const double rf = sqrt((double)far_distance2(fw, t, &diag));
+    if (!(rf > 0.0)) return 4;
+    // a shell about the brick, from Rf outside it to rc from its far corners
+    const double in = rf + diag / 4.0, out = sqrt(fw.rc2) - diag / 2.0;
+    const double far_atoms =
+        4.18879 * (out * out * out - in * in * in) * fw.n_atoms / std::max(fw.volume, 1e-9);
+    if (!(far_atoms >= 32.0)) return 4;
+    const int64_t bricks = (int64_t)((nx + 15) / 16) * ((ny + 7) / 8) * ((nz + 15) / 16);
+    const double h = std::max(fw.cell_len[0] / (nx - 1), fw.cell_len[2] / (nz - 1));
+    const int64_t slots = 3 * ctx->num_sms;
+    return bricks >= (h <= 0.14 ? slots / 2 : slots) ? 8 : 4;
+}
+
 int fill_grid_task(er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, float* out,
                    GridTask& t, int tile_p) {
     if (tile_p != 4 && tile_p != 8)
@@ -248,6 +298,7 @@ int fill_grid_task(er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, floa
     t.nb[0] = (nx + 2 * tile_p - 1) / (2 * tile_p);
     t.nb[1] = (ny + 2 * kWJ - 1) / (2 * kWJ);
     t.nb[2] = (nz + 2 * kWK - 1) / (2 * kWK);
+    t.far2 = far_distance2(fw, t);
     t.out = out;
     t.out64 = nullptr;
     return ER_OK;
@@ -682,11 +733,12 @@ int er_grid(er_ctx* ctx, int fw_id, int nx, int ny, int nz, int flags, void* out
     ER_CUDA(ctx, cudaSetDevice(ctx->device));
     const FwRecord* f = find_fw(ctx, fw_id);
     if (!f) return set_error(ctx, ER_ERR_NOT_FOUND, "grid: unknown framework id");
-    const int tile_p = (flags & ER_TILE_P8) ? 8 : 4;
-    const int prec = (flags & ER_COUNT_PAIRS) ? PREC_COUNT
+    const int prec = (flags & ER_COUNT_PAIRS)  ? PREC_COUNT
                      : (flags & ER_PREC_FP32) ? PREC_FP32
                      : (flags & ER_PREC_COMP) ? PREC_COMP
+                     : (flags & ER_PREC_FP64) ? PREC_FP64
                                               : PREC_NEAR64;
+    const int tile_p = (flags & ER_TILE_P8) ? 8 : default_tile(ctx, *f, nx, ny, nz, prec);
     const size_t npts = (size_t)nx * ny * nz;
     const bool dev_out = (flags & ER_OUT_DEVICE) != 0;
     const bool f64 = (flags & ER_OUT_F64) != 0;
@@ -856,7 +908,11 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
         }
         int tile_p = 4;
         int st = ER_OK;
-        if (autotune && jobs[i].nx >= 2 && jobs[i].ny >= 2 && jobs[i].nz >= 2)
+        const bool dims_ok = jobs[i].nx >= 2 && jobs[i].ny >= 2 && jobs[i].nz >= 2;
+        if (dims_ok)
+            tile_p = default_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, prec);
+        // (a far field needs P = 8 and always pays: nothing to time)
+        if (autotune && dims_ok && tile_p == 4)
             st = tune_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device, prec,
                            &tile_p);
         GridTask t;

@@ -182,9 +182,13 @@ CutoffConsts make_cutoff_consts(double rc2, double box_diag, double r2min);
 // Grid dimensions accepted by every grid entry point: each >= 2 (axes
 // i / (N - 1)) and at most 4e9 points; checked before any allocation.
 int check_grid_dims(er_ctx* ctx, int nx, int ny, int nz, const char* who);
+// Kernel variant (points per thread) of a grid where the caller asks for none:
+// the same for a single call, a batch, the server and a Widom batch, so that
+// their results are equal bit for bit.
+int default_tile(const er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, int prec);
 // Fills a grid task (validates dims) and launches the plain grid kernel on `st`.
 int fill_grid_task(er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, float* out,
-                   GridTask& t, int tile_p = 4);
+                   GridTask& t, int tile_p);
 int launch_grid_plain_on(er_ctx* ctx, const GridTask& t, int prec, cudaStream_t st);
 // Widom pipeline on stream `st` with scratch `hs`; when host_out (pinned) is
 // given, the reduction and the blocked count are copied there asynchronously.

@@ -772,7 +772,8 @@ int henry_one(er_ctx* ctx, HenryPipe& P, const FwRecord& fw, double temperature,
             P.mask.ensure_on(pts, ctx->pool, st))
             return set_error(ctx, ER_ERR_NOMEM, "henry batch: grid/mask allocation failed");
         GridTask t;
-        int s = fill_grid_task(ctx, fw, bd[0], bd[1], bd[2], (float*)P.grid.ptr, t, 4);
+        const int tile = default_tile(ctx, fw, bd[0], bd[1], bd[2], PREC_NEAR64);
+        int s = fill_grid_task(ctx, fw, bd[0], bd[1], bd[2], (float*)P.grid.ptr, t, tile);
         if (s == ER_OK) s = launch_grid_plain_on(ctx, t, PREC_NEAR64, st);
         if (s == ER_OK)
             s = block_pockets_device_on(ctx, P.ps, st, (const float*)P.grid.ptr, bd[0], bd[1],

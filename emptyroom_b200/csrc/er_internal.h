@@ -51,6 +51,8 @@ struct GridTask {
     int nx, ny, nz;
     int nb[3];          // bricks per axis
     int tile_p;         // points per thread of the kernel variant (brick 2P x 8 x 16)
+    float far2;         // squared distance from which on a brick's atoms are interpolated
+                        // (0: none)
     float* out;         // nx*ny*nz, index k + j*nz + i*ny*nz
     double* out64;      // same layout, FP64 (PREC_FP64 jobs only)
 };

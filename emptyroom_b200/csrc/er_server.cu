@@ -320,7 +320,9 @@ struct er_server {
                 st = ER_ERR_NOMEM;
             } else {
                 er::GridTask t;
-                st = er::fill_grid_task(ctx, *fr, job.nx, job.ny, job.nz, g.ptr, t);
+                st = er::fill_grid_task(ctx, *fr, job.nx, job.ny, job.nz, g.ptr, t,
+                                        er::default_tile(ctx, *fr, job.nx, job.ny, job.nz,
+                                                         er::PREC_NEAR64));
                 if (st == ER_OK) st = er::launch_grid_plain_on(ctx, t, er::PREC_NEAR64, sl.stream);
                 if (st == ER_OK && job.grid_out_host &&
                     cudaMemcpyAsync(job.grid_out_host, g.ptr, g.bytes, cudaMemcpyDeviceToHost,

@@ -107,7 +107,8 @@ int er_framework_bytes(er_ctx* ctx, int fw_id, size_t* bytes);
                                 point instead of the energy (same traversal) */
 #define ER_TILE_P8 0x80      /* kernel variant with 8 points per thread (16 x 8 x 16
                                 bricks) instead of 4; results agree within the FP32
-                                tolerance, not bit for bit */
+                                tolerance, not bit for bit. Fine grids of the default
+                                precision run it without being asked */
 
 /* Energies above this value (K) are written as this value (overflow cap). */
 #define ER_ENERGY_CAP 1.0e30

@@ -248,6 +248,50 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const int* __r
     }
 }
 
+// The same by one CTA, four entries per thread and turn, for tables that take a
+// few turns: one launch instead of three.
+constexpr int kScanSmall = 16384;
+
+__global__ void __launch_bounds__(1024) scan_small_kernel(const int* __restrict__ in, int n,
+                                                          int* __restrict__ out) {
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < n; base += 4096) {
+        const int i = base + 4 * (int)threadIdx.x;
+        int v[4], s = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = i + k < n ? in[i + k] : 0;
+            s += v[k];
+        }
+        int x = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[w] = x;
+        __syncthreads();
+        int below = 0, total = 0;
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+            const int c = wsum[k];
+            below += k < w ? c : 0;
+            total += c;
+        }
+        int run = carry + below + x - s;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i + k < n) out[i + k] = run;
+            run += v[k];
+        }
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
 int scan_tiles(int n) { return (n + kScanTile - 1) / kScanTile; }
 
 int scan_exclusive(er_ctx* ctx, const int* in, int n, int* out, int* tile_sums,
@@ -335,13 +379,35 @@ __global__ void henry_place_kernel(const int* __restrict__ n_valid, const int* _
     }
 }
 
-// One warp per warp boundary m * warp_pts (m >= 1) below n_valid, after
-// henry_place_kernel: the bin holding that position (binary search of the bin
-// starts); when the boundary cuts it and is the first boundary to do so, the
+// Scatter and placement in one, for runs up to kFusedPlaceN: writing the 24-byte
+// points at random into the L2 costs less than a second launch there (call of
+// 32k insertions 93 against 99 us, 100k 109 / 112), and more from there on (400k
+// 180 / 175, 1e6 307 / 296, 1e7 2600 / 1650).
+constexpr int kFusedPlaceN = 1 << 18;
+
+__global__ void henry_scatter_place_kernel(const int* __restrict__ key,
+                                           const int* __restrict__ slot, int n,
+                                           const int* __restrict__ starts, uint64_t seed, Frame fr,
+                                           int* __restrict__ tmp, int* __restrict__ order,
+                                           double* __restrict__ pts) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int k = key[i];
+    if (k < 0) return;
+    const int at = starts[k] + slot[i];
+    tmp[at] = i;
+    order[at] = i;
+    put_point(seed, fr, i, pts + 3 * (size_t)at);
+}
+
+// One warp per warp boundary m * warp_pts (m >= 1) below n_valid, after the
+// placement: the bin holding that position (the key of the insertion there);
+// when the boundary cuts it and is the first boundary to do so, the
 // warp rewrites the bin in ascending insertion order (each entry's rank among
 // the bin's entries, compared 32 at a time through shuffles).
 __global__ void henry_order_straddling_kernel(const int* __restrict__ starts, int n_keys,
-                                              int warp_pts, const int* __restrict__ tmp,
+                                              const int* __restrict__ key, int warp_pts,
+                                              const int* __restrict__ tmp,
                                               uint64_t seed, Frame fr, int* __restrict__ order,
                                               double* __restrict__ pts) {
     const int lane = threadIdx.x & 31;
@@ -349,14 +415,8 @@ __global__ void henry_order_straddling_kernel(const int* __restrict__ starts, in
     const long long qb = m * warp_pts;
     if (qb >= starts[n_keys]) return;
     const int q = (int)qb;
-    // the last bin b with starts[b] <= q: q lies in [starts[b], starts[b + 1])
-    int lo = 0, hi = n_keys - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (starts[mid] <= q) lo = mid;
-        else hi = mid - 1;
-    }
-    const int s = starts[lo], L = starts[lo + 1] - s;
+    const int bin = key[tmp[q]];
+    const int s = starts[bin], L = starts[bin + 1] - s;
     if (s == q || q - warp_pts > s) return;  // not cut here, or cut first by an earlier boundary
     for (int q0 = 0; q0 < L; q0 += 32) {
         const int i = q0 + lane;
@@ -407,10 +467,15 @@ __device__ __forceinline__ Lse lse_tree(Lse v, Lse* sm) {
 // Block b sums insertions [b*chunk, (b+1)*chunk) (thread t: b*chunk + t + 256 k).
 // neg_inv_t = -1 / T: the exponent -E / T of src/doHenry.h:107 as a product
 // (within an ulp of the quotient; the Boltzmann factor moves by ~1e-15 relative).
+// The block that finishes last merges the blocks' sums in a fixed order and
+// writes the result (a launch of its own for that took 6 us).
 __global__ void __launch_bounds__(256) henry_reduce_kernel(const float* __restrict__ E, int n,
                                                            double neg_inv_t, int chunk,
-                                                           Lse* __restrict__ part) {
+                                                           Lse* __restrict__ part, int* done,
+                                                           const int* __restrict__ n_blocked,
+                                                           HenryOut* __restrict__ out) {
     __shared__ Lse sm[256];
+    __shared__ int is_last;
     const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
     // two passes over this thread's entries: the largest exponent, then the
     // weights exp(x - m), which do not wait for one another (with a running
@@ -434,18 +499,27 @@ __global__ void __launch_bounds__(256) henry_reduce_kernel(const float* __restri
         }
     }
     const Lse r = lse_tree(acc, sm);
-    if (threadIdx.x == 0) part[blockIdx.x] = r;
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = r;
+        __threadfence();
+        is_last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    Lse all{-INFINITY, 0.0, 0.0};
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) {
+        const double* p = reinterpret_cast<const double*>(part + i);
+        all = lse_merge(all, Lse{__ldcg(p), __ldcg(p + 1), __ldcg(p + 2)});
+    }
+    const Lse t = lse_tree(all, sm);
+    if (threadIdx.x == 0) {
+        out->lse[0] = t.m;
+        out->lse[1] = t.s;
+        out->lse[2] = t.se;
+        out->n_blocked = *n_blocked;
+    }
 }
-
-__global__ void __launch_bounds__(256) henry_final_kernel(const Lse* __restrict__ part, int nb,
-                                                          Lse* __restrict__ out) {
-    __shared__ Lse sm[256];
-    Lse acc{-INFINITY, 0.0, 0.0};
-    for (int i = threadIdx.x; i < nb; i += 256) acc = lse_merge(acc, part[i]);
-    const Lse r = lse_tree(acc, sm);
-    if (threadIdx.x == 0) *out = r;
-}
-
 
 int henry_reserve(er_ctx* ctx, HenryScratch& hs, int64_t n, cudaStream_t st) {
     const size_t N = (size_t)n;
@@ -487,12 +561,11 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
         hs.bin.ensure_on(N * sizeof(int), pool, st) ||
         hs.order.ensure_on(N * sizeof(int), pool, st) ||
         hs.tmp.ensure_on(N * sizeof(int), pool, st) ||
-        hs.counts.ensure_on(2 * (size_t)g.n_keys * sizeof(int), pool, st) ||
+        hs.counts.ensure_on((2 * (size_t)g.n_keys + 2) * sizeof(int), pool, st) ||
         hs.starts.ensure_on(((size_t)g.n_keys + 1) * sizeof(int), pool, st) ||
         hs.e.ensure_on(N * sizeof(float), pool, st) ||
-        hs.nblk.ensure_on(4 * sizeof(int), pool, st) ||
         hs.part.ensure_on(4096 * sizeof(Lse), pool, st) ||
-        hs.res.ensure_on(sizeof(Lse), pool, st))
+        hs.res.ensure_on(sizeof(HenryOut), pool, st))
         return set_error(ctx, ER_ERR_NOMEM, "henry: device scratch allocation failed");
     const uint8_t* d_mask = nullptr;
     if (block_mask) {
@@ -511,18 +584,19 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
         }
     }
     int* counts = (int*)hs.counts.ptr;
-    int* tsum = counts + g.n_keys;  // tile sums of the scan
+    int* nblk = counts + g.n_keys;  // blocked insertions, and reduction blocks that are done
+    int* rdone = nblk + 1;
+    int* tsum = nblk + 2;           // tile sums of the scan
     int* starts = (int*)hs.starts.ptr;
-    int* nblk = (int*)hs.nblk.ptr;
     float* E = (float*)hs.e.ptr;
-    ER_CUDA(ctx, cudaMemsetAsync(counts, 0, (size_t)g.n_keys * sizeof(int), st));
-    ER_CUDA(ctx, cudaMemsetAsync(nblk, 0, sizeof(int), st));
+    ER_CUDA(ctx, cudaMemsetAsync(counts, 0, ((size_t)g.n_keys + 2) * sizeof(int), st));
     const int gthreads = 256;
     const int gblocks = (int)std::min<int64_t>((n + gthreads - 1) / gthreads,
                                                (int64_t)ctx->num_sms * 32);
-    // the slot of each insertion in its bin goes to `order` until the sort
-    // overwrites it with the sorted insertion indices
-    int* slot = (int*)hs.order.ptr;
+    // the slot of each unblocked insertion in its bin waits where its energy
+    // goes; the sorted insertion indices
+    int* slot = (int*)hs.e.ptr;
+    int* sorted = (int*)hs.order.ptr;
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[0], st));
     MaskGeom mg{};
     const uint8_t* d_cell = nullptr;
@@ -542,7 +616,9 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
     }
     henry_gen_kernel<<<gblocks, gthreads, 0, st>>>(seed, n, g, d_cell, mg, (int*)hs.bin.ptr, slot,
                                                    counts, E, nblk);
-    {
+    if (g.n_keys <= kScanSmall) {
+        scan_small_kernel<<<1, 1024, 0, st>>>(counts, g.n_keys, starts);
+    } else {
         const int tiles = (g.n_keys + kScanTile - 1) / kScanTile;
         scan_tiles_kernel<<<tiles, kScanThreads, 0, st>>>(counts, g.n_keys, tsum);
         scan_top_kernel<<<1, 1024, 0, st>>>(tsum, tiles, starts + g.n_keys);
@@ -556,26 +632,31 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
     const int sblocks = (int)std::min<int64_t>(((int64_t)n + 4 * gthreads - 1) / (4 * gthreads),
                                                1 << 20);
     const int pblocks = (int)std::min<int64_t>(((int64_t)n + gthreads - 1) / gthreads, 1 << 20);
-    henry_scatter_kernel<<<sblocks, gthreads, 0, st>>>((const int*)hs.bin.ptr, slot, n, starts,
-                                                       (int*)hs.tmp.ptr);
     Frame fr;
     for (int k = 0; k < 9; ++k) fr.r[k] = fw.dev.r[k];
-    henry_place_kernel<<<pblocks, gthreads, 0, st>>>(starts + g.n_keys, (const int*)hs.tmp.ptr,
-                                                      seed, fr, (int*)hs.order.ptr,
-                                                      (double*)hs.pts.ptr);
+    if (n <= kFusedPlaceN) {
+        henry_scatter_place_kernel<<<(n + gthreads - 1) / gthreads, gthreads, 0, st>>>(
+            (const int*)hs.bin.ptr, slot, n, starts, seed, fr, (int*)hs.tmp.ptr, sorted,
+            (double*)hs.pts.ptr);
+    } else {
+        henry_scatter_kernel<<<sblocks, gthreads, 0, st>>>((const int*)hs.bin.ptr, slot, n, starts,
+                                                           (int*)hs.tmp.ptr);
+        henry_place_kernel<<<pblocks, gthreads, 0, st>>>(starts + g.n_keys, (const int*)hs.tmp.ptr,
+                                                          seed, fr, sorted, (double*)hs.pts.ptr);
+    }
     const int warp_pts = 32 * henry_points_per_thread(n);
     const int64_t n_bounds = ((int64_t)n - 1) / warp_pts;  // boundaries below n
     if (n_bounds > 0)
         henry_order_straddling_kernel<<<(int)((n_bounds + 7) / 8), 256, 0, st>>>(
-            starts, g.n_keys, warp_pts, (const int*)hs.tmp.ptr, seed, fr, (int*)hs.order.ptr,
-            (double*)hs.pts.ptr);
+            starts, g.n_keys, (const int*)hs.bin.ptr, warp_pts, (const int*)hs.tmp.ptr, seed, fr,
+            sorted, (double*)hs.pts.ptr);
     ER_CUDA(ctx, cudaGetLastError());
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[2], st));
     PointTask task;
     task.fw = fw.dev;
     task.cc = make_cutoff_consts(fw.rc2, 0.0, 1e-16 * 1e-16);  // min_r, src/doHenry.h:15
     task.pts = (const double*)hs.pts.ptr;
-    task.order = (const int*)hs.order.ptr;
+    task.order = sorted;
     task.seed = seed;
     task.n_valid = starts + g.n_keys;
     task.energies = E;
@@ -601,19 +682,17 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
     else ER_CUDA(ctx, energy(henry_energy_kernel<kHenryPSmall, 1>, 1));
     ER_CUDA(ctx, cudaGetLastError());
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[3], st));
+    // at least 2048 insertions a block: fewer partial sums to merge
     const int rblocks = std::min(4096, std::max(1, ctx->num_sms * 4));
-    const int chunk = (n + rblocks - 1) / rblocks;
+    const int chunk = std::max((n + rblocks - 1) / rblocks, 2048);
     const int nrb = (n + chunk - 1) / chunk;
-    henry_reduce_kernel<<<nrb, 256, 0, st>>>(E, n, -1.0 / temperature, chunk, (Lse*)hs.part.ptr);
-    henry_final_kernel<<<1, 256, 0, st>>>((const Lse*)hs.part.ptr, nrb, (Lse*)hs.res.ptr);
+    henry_reduce_kernel<<<nrb, 256, 0, st>>>(E, n, -1.0 / temperature, chunk, (Lse*)hs.part.ptr,
+                                             rdone, nblk, (HenryOut*)hs.res.ptr);
     ER_CUDA(ctx, cudaGetLastError());
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[4], st));
-    if (host_out) {
-        ER_CUDA(ctx, cudaMemcpyAsync(host_out->lse, hs.res.ptr, sizeof(Lse),
+    if (host_out)
+        ER_CUDA(ctx, cudaMemcpyAsync(host_out, hs.res.ptr, sizeof(HenryOut),
                                      cudaMemcpyDeviceToHost, st));
-        ER_CUDA(ctx, cudaMemcpyAsync(&host_out->n_blocked, nblk, sizeof(int),
-                                     cudaMemcpyDeviceToHost, st));
-    }
     return ER_OK;
 }
 
@@ -657,15 +736,17 @@ extern "C" int er_henry(er_ctx* ctx, int fw_id, double temperature, int64_t n_in
     if (!f) return set_error(ctx, ER_ERR_NOT_FOUND, "henry: unknown framework id");
     int st = henry_check(ctx, temperature, n_ins, block_mask, mnx, mny, mnz);
     if (st != ER_OK) return st;
-    HenryOut h;
+    if (ctx->henry.host.ensure(sizeof(HenryOut)) != ER_OK)
+        return set_error(ctx, ER_ERR_NOMEM, "henry: pinned staging failed");
+    HenryOut* h = (HenryOut*)ctx->henry.host.ptr;
     st = henry_enqueue(ctx, *f, temperature, (int)n_ins, seed, block_mask, mnx, mny, mnz,
-                       ctx->stream, ctx->henry, &h);
+                       ctx->stream, ctx->henry, h);
     if (st != ER_OK) return st;
     if (energies_out)
         ER_CUDA(ctx, cudaMemcpyAsync(energies_out, ctx->henry.e.ptr, (size_t)n_ins * sizeof(float),
                                      cudaMemcpyDeviceToHost, ctx->stream));
     ER_SYNC(ctx, ctx->stream);
-    henry_finish(h, n_ins, temperature, out);
+    henry_finish(*h, n_ins, temperature, out);
     return ER_OK;
 }
 

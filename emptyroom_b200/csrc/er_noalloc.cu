@@ -141,7 +141,7 @@ extern "C" int er_henry_stats_noalloc(er_ctx* ctx, const float* energies, int64_
     noalloc::Stats* scratch = nullptr;
     int st = noalloc::scratch_for(ctx, &scratch);
     if (st != ER_OK) return st;
-    // the block partition of er_henry's reduction (4 blocks per SM, at most
+    // the block partition of er_henry's reduction of long runs (4 blocks per SM, at most
     // kSlots), computed in 64-bit so that it cannot overflow at the top of the range
     const int64_t rblocks = std::min<int64_t>(noalloc::kSlots, std::max(1, ctx->num_sms * 4));
     const int64_t chunk = (n + rblocks - 1) / rblocks;

@@ -1,0 +1,28 @@
+"""Widom runs where the layout of the insertions changes its kernels (one-CTA and
+tiled scan of the bin counts, one or two placement passes, one or several
+reduction blocks), with and without a pocket mask: K_H against the oracle."""
+import numpy as np
+import pytest
+
+import oracle
+from emptyroom_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+T = 310.0
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 1 << 18, (1 << 18) + 1])
+@pytest.mark.parametrize("masked", [False, True])
+def test_widom_layout_paths(ctx, n, masked):
+    f = synth.config1(12)
+    P = f.particles()
+    fw = ctx.upload(P, f.t_matrix, f.rep, f.rc2)
+    mask = (np.random.default_rng(n).random((17, 15, 19)) < 0.02).astype(np.uint8) if masked else None
+    r = ctx.henry(fw, T, n, seed=77, block_mask=mask)
+    again = ctx.henry(fw, T, n, seed=77, block_mask=mask)
+    fw.release()
+    assert r == again
+    o = oracle.henry(P, f.t_matrix, f.rep, f.rc2, T, 77, n, mask=mask)
+    assert r["n_blocked"] == o["n_blocked"] and r["n_insertions"] == n
+    assert abs(r["sum_w"] - o["sum_w"]) <= 1e-6 * o["sum_w"]

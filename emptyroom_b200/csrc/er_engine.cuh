@@ -78,11 +78,20 @@ struct PrecTraits {
     static constexpr int inner_chunk = PREC == PREC_NEAR64 ? 16 : 64;
 };
 
-// The same where a brick has a far field, for its nodes and for what is left of
-// the inner lists: with 16 the mean error on E < -10 K points was within 3 % of
-// the one without a far field, either way; with 8 it is 4-10 % below it (five
-// cells at 0.1-0.155 A), for 2 % more time.
-constexpr int kFarChunk = 8;
+// The same for two policies whose other choices would raise the error a little.
+// Where a brick has a far field, for its nodes and for what is left of the inner
+// lists: with 16 the mean error on E < -10 K points was within 3 % of the one
+// without a far field, either way; with 8 it is 4-10 % below it (five cells at
+// 0.1-0.155 A), for 2 % more time. And for Widom warps of 128 points, whose boxes
+// have fewer atoms within kNearR than those of 256: with 16 the mean error of 1.5e6
+// insertions was 12 % above that of 256-point warps, with 8 it is 3.5 % above it
+// and 2-4 % below it at 1.2e6, 2e5 and 32768.
+constexpr int kShortChunk = 8;
+template <class Pol, int PREC>
+struct InnerChunk {
+    static constexpr int value =
+        PREC == PREC_NEAR64 && Pol::kShort ? kShortChunk : PrecTraits<PREC>::inner_chunk;
+};
 constexpr int kNearCap = 256;     // near-list capacity per warp (overflow stays FP32)
 constexpr int kRec = 3;           // borderline shell atoms recorded per thread and flush
                                   // (10-bit list positions packed in one register)
@@ -460,6 +469,7 @@ struct GridPolicy : BrickPart<SPLIT> {
     // interpolated, 0 for none. Bricks with less than half their points on the
     // grid do without: the nodes would cost more than the points.
     static constexpr bool kFar = P_ == 8 && SPLIT == 1;
+    static constexpr bool kShort = kFar;
     __device__ __forceinline__ float far_from2() const {
         const int ni = min(kBI, T->nx - i0), nj = min(kBJ, T->ny - j0), nk = min(kBK, T->nz - k0);
         return 2 * ni * nj * nk >= kBI * kBJ * kBK ? T->far2 : 0.f;
@@ -501,6 +511,7 @@ struct PointPolicy : BrickPart<SPLIT> {
     static constexpr int kP = P_ / SPLIT;
     static constexpr int kBoxP = P_;  // points per lane of the box passes
     static constexpr bool kFar = false;
+    static constexpr bool kShort = P_ == 4;  // (shared by its split forms)
     static constexpr bool kLattice = false;
     static_assert(P_ % SPLIT == 0 && kWarps % SPLIT == 0, "whole points and warps");
     const PointTask* T;
@@ -647,8 +658,7 @@ __device__ __forceinline__ void lattice_inner(EngineSmem& s, const unsigned shor
                                               int n_in, Lane<Pol, PREC>& L) {
     constexpr int M = Pol::kP / 2;
     constexpr bool kComp = PrecTraits<PREC>::comp;
-    constexpr int kChunk =
-        Pol::kFar && PrecTraits<PREC>::far ? kFarChunk : PrecTraits<PREC>::inner_chunk;
+    constexpr int kChunk = InnerChunk<Pol, PREC>::value;
     f2_t px2[M], acc2[M];
     double acc64[2 * M];
 #pragma unroll
@@ -836,9 +846,7 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
     const char* cbase = reinterpret_cast<const char*>(s.cand);
     int nrec = 0;
     rec = 0;
-    auto inner_atom = [&](unsigned off) {
-        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(cbase + off);       // x x | y z
-        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(cbase + off + 16);  // C12 | -C6
+    auto inner_atom = [&](const ulonglong2 v0, const ulonglong2 v1) {  // x x | y z, C12 | -C6
         if (PREC == PREC_COUNT) {
 #pragma unroll
             for (int m = 0; m < M; ++m) acc2[m] = f2_add(acc2[m], one2);
@@ -860,9 +868,8 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
             acc2[m] = f2_fma(u3, f2_fma(v1.x, u3, v1.y), acc2[m]);
         }
     };
-    auto shell_atom = [&](unsigned off, int q) {
-        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(cbase + off);
-        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(cbase + off + 16);
+    // returns the atom's smallest |r^2 - fl32(rc^2)|
+    auto shell_atom = [&](const ulonglong2 v0, const ulonglong2 v1) {
         float ay, az;
         f2_unpack(v0.y, ay, az);
         const f2_t ay2 = f2_pack(ay, ay), az2 = f2_pack(az, az);
@@ -886,9 +893,39 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
                 acc2[m] = f2_fma(f2_mul(u3, in), f2_fma(v1.x, u3, v1.y), acc2[m]);
             }
         }
-        if (mn <= win) {  // rare: a pair of this atom sits near the cutoff
-            rec = (rec << 10) | (unsigned)q;
-            ++nrec;
+        return mn;
+    };
+    auto load = [&](unsigned off, ulonglong2& v0, ulonglong2& v1) {
+        v0 = *reinterpret_cast<const ulonglong2*>(cbase + off);
+        v1 = *reinterpret_cast<const ulonglong2*>(cbase + off + 16);
+    };
+    auto inner = [&](auto n_, const unsigned short* l) {
+        constexpr int N = decltype(n_)::value;
+        ulonglong2 v0[N], v1[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) load(l[k], v0[k], v1[k]);
+#pragma unroll
+        for (int k = 0; k < N; ++k) inner_atom(v0[k], v1[k]);
+    };
+    // N atoms (positions q .. q + N - 1 of the list): one branch for them all
+    auto shell = [&](auto n_, int q) {
+        constexpr int N = decltype(n_)::value;
+        ulonglong2 v0[N], v1[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) load(wl[kMaxCand - 1 - q - k], v0[k], v1[k]);
+        float mn[N], all = INFINITY;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            mn[k] = shell_atom(v0[k], v1[k]);
+            all = fminf(all, mn[k]);
+        }
+        if (all <= win) {  // rare: a pair of these atoms sits near the cutoff
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                if (mn[k] <= win) {
+                    rec = (rec << 10) | (unsigned)(q + k);
+                    ++nrec;
+                }
         }
     };
     int q = 0;
@@ -897,23 +934,13 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
     double acc64[2 * M];
 #pragma unroll
     for (int m = 0; m < 2 * M; ++m) acc64[m] = 0.0;
+    // atoms whose records are loaded together: as many as the registers hold
+    constexpr int kIn = M > 2 ? 4 : 8, kSh = M > 2 ? 2 : 4;
     while (q < n_in) {
-        const int qe = kComp ? min(q + PrecTraits<PREC>::inner_chunk, n_in) : n_in;
-        // four atoms per iteration: sixteen independent FP32 chains for the
-        // scheduler (the kernel is latency-bound at two CTAs per SM); with two
-        // shell atoms per iteration and the register fold, 1.247 -> 1.207 ms
-        // per 1e7 insertions on a config-1 cell
-        for (; q + 3 < qe; q += 4) {
-            inner_atom(wl[q]);
-            inner_atom(wl[q + 1]);
-            inner_atom(wl[q + 2]);
-            inner_atom(wl[q + 3]);
-        }
-        for (; q + 1 < qe; q += 2) {
-            inner_atom(wl[q]);
-            inner_atom(wl[q + 1]);
-        }
-        if (q < qe) inner_atom(wl[q++]);
+        const int qe = kComp ? min(q + InnerChunk<Pol, PREC>::value, n_in) : n_in;
+        for (; q + kIn <= qe; q += kIn) inner(Int<kIn>{}, wl + q);
+        for (; q + 2 <= qe; q += 2) inner(Int<2>{}, wl + q);
+        if (q < qe) inner(Int<1>{}, wl + q++);
         if (kComp) fold_regs<M>(acc64, acc2);
     }
     if (kComp) {
@@ -923,11 +950,8 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
     q = 0;
     while (q < n_sh) {
         const int qe = kComp ? min(q + kAccChunk, n_sh) : n_sh;
-        for (; q + 1 < qe; q += 2) {
-            shell_atom(wl[kMaxCand - 1 - q], q);
-            shell_atom(wl[kMaxCand - 2 - q], q + 1);
-        }
-        for (; q < qe; ++q) shell_atom(wl[kMaxCand - 1 - q], q);
+        for (; q + kSh <= qe; q += kSh) shell(Int<kSh>{}, q);
+        for (; q < qe; ++q) shell(Int<1>{}, q);
         if (kComp) fold_packed<M>(s, acc2);
     }
     if (!kComp) fold_packed<M>(s, acc2);
@@ -973,7 +997,7 @@ __device__ __forceinline__ int single_lists(EngineSmem& s, const unsigned short*
     double acc64 = 0.0;
     int q = 0;
     while (q < n_in) {
-        const int qe = kComp ? min(q + PrecTraits<PREC>::inner_chunk, n_in) : n_in;
+        const int qe = kComp ? min(q + InnerChunk<Pol, PREC>::value, n_in) : n_in;
         for (; q + kBatch <= qe; q += kBatch) inner(Int<kBatch>{}, wl + q);
         for (; q < qe; ++q) inner(Int<1>{}, wl + q);
         if (kComp || Pol::kLattice) {
@@ -1329,7 +1353,7 @@ template <class Pol, int PREC>
 __device__ __forceinline__ void far_field(EngineSmem& s, const Pol& pol, const FwDev& fw,
                                           int n_far) {
     constexpr int M = kFarN / 2;
-    constexpr int kChunk = kFarChunk;
+    constexpr int kChunk = kShortChunk;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     FarSmem& f = *reinterpret_cast<FarSmem*>(&s.wl[0][0]);
     // this warp's share of the atoms

@@ -9,7 +9,7 @@
 //      position's point, then order the bins that straddle a warp boundary by
 //      insertion index (so every warp's point set, and with it every FP32
 //      rounding, is deterministic)
-//   5. energy  the shared LJ engine over 2048 (1024 for runs below 1e6)
+//   5. energy  the shared LJ engine over 2048 (1024 for runs below 1.5 * 2^20)
 //              points per CTA, in bin order
 //   6. reduce  FP64 log-sum-exp of exp(-E/T) and E exp(-E/T) in insertion
 //              order with a fixed tree: (m, s, se) with sum w = s e^m.
@@ -26,13 +26,15 @@
 
 namespace er {
 
-// Insertions per thread of the energy kernel: 8 for large runs (1.82 against
-// 2.00 ms per 1e7 insertions on a config-1 cell); 4 below kHenrySmallN, where
-// a run fills few waves of CTAs and more, smaller CTAs finish sooner (0.16
-// against 0.26 ms for 1e5 insertions).
+// Insertions per thread of the energy kernel: 4 below kHenrySmallN, where a run
+// fills few waves of CTAs, whose more numerous and smaller halves finish sooner,
+// and where its points lie so far apart that a smaller CTA reaches fewer atoms;
+// 8 from there on, each atom loaded serving twice the points. Measured 8 / 4, us
+// a call: 1e6 insertions 297 / 275 (cell of 424 atoms), 835 / 698 (1500 atoms);
+// 2e6 433 / 448; 3e6 571 / 595; 1e7 1650 / 1800.
 constexpr int kHenryP = 8;
 constexpr int kHenryPSmall = 4;
-constexpr int64_t kHenrySmallN = 1000000;
+constexpr int64_t kHenrySmallN = 3 << 19;
 inline int henry_points_per_thread(int64_t n) { return n < kHenrySmallN ? kHenryPSmall : kHenryP; }
 
 struct BinGeom {

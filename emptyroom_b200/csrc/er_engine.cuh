@@ -949,7 +949,7 @@ __device__ __forceinline__ int generic_packed_lists(EngineSmem& s, const unsigne
     return nrec;
 }
 
-// Inner and shell lists of a lane's one point (split bricks), kBatch atoms at a
+// Inner and shell lists of a lane's one point (split bricks), several atoms at a
 // time. Per point the same operations in the same order as the packed forms
 // above, so the energies are theirs bit for bit.
 template <class Pol, int PREC>
@@ -957,7 +957,11 @@ __device__ __forceinline__ int single_lists(EngineSmem& s, const unsigned short*
                                             int n_sh, float rc2f, float win,
                                             Lane<Pol, PREC>& L, unsigned& rec) {
     constexpr bool kComp = PrecTraits<PREC>::comp;
-    constexpr int kBatch = 4;
+    // one point's state leaves the registers for many records, and two warps per
+    // scheduler need them (32^3 grid, records loaded together: 4 34.9 us, 8 32.4, 16
+    // 30.8)
+    constexpr int kSh = 16;
+    constexpr int kIn = InnerChunk<Pol, PREC>::value < 16 ? InnerChunk<Pol, PREC>::value : 16;
     const float px = L.px[0], py = L.py[0], pz = L.pz[0];
     const char* cbase = reinterpret_cast<const char*>(s.cand);
     float acc = 0.f;
@@ -989,8 +993,9 @@ __device__ __forceinline__ int single_lists(EngineSmem& s, const unsigned short*
     int q = 0;
     while (q < n_in) {
         const int qe = kComp ? min(q + InnerChunk<Pol, PREC>::value, n_in) : n_in;
-        for (; q + kBatch <= qe; q += kBatch) inner(Int<kBatch>{}, wl + q);
-        for (; q < qe; ++q) inner(Int<1>{}, wl + q);
+        for (; q + kIn <= qe; q += kIn) inner(Int<kIn>{}, wl + q);
+        for (; q + 2 <= qe; q += 2) inner(Int<2>{}, wl + q);
+        if (q < qe) inner(Int<1>{}, wl + q++);
         if (kComp || Pol::kLattice) {
             acc64 += (double)acc;
             acc = 0.f;
@@ -1031,7 +1036,8 @@ __device__ __forceinline__ int single_lists(EngineSmem& s, const unsigned short*
     q = 0;
     while (q < n_sh) {
         const int qe = kComp ? min(q + kAccChunk, n_sh) : n_sh;
-        for (; q + kBatch <= qe; q += kBatch) shell(Int<kBatch>{}, q);
+        for (; q + kSh <= qe; q += kSh) shell(Int<kSh>{}, q);
+        for (; q + 4 <= qe; q += 4) shell(Int<4>{}, q);
         for (; q < qe; ++q) shell(Int<1>{}, q);
         if (kComp) {
             tot_at(s, 0) += (double)acc;
@@ -1457,53 +1463,65 @@ __device__ __forceinline__ void warp_flush(EngineSmem& s, const Pol& pol, const 
     const float rnear2 = kNearR * kNearR;
     const float wl0x = s.wbox[w][0], wl0y = s.wbox[w][1], wl0z = s.wbox[w][2];
     const float wh0x = s.wbox[w][3], wh0y = s.wbox[w][4], wh0z = s.wbox[w][5];
-    for (int base = 0; base < n_cand; base += 32) {
-        const int c = base + lane;
-        bool in = false, sh = false, nr = false;
-        if (c < n_cand) {
-            const float4 a = *reinterpret_cast<const float4*>(&s.cand[c].ax);
-            const float ax = a.x, ay = a.z, az = a.w;
-            const float ex = fmaxf(0.f, fmaxf(wl0x - ax, ax - wh0x));
-            const float ey = fmaxf(0.f, fmaxf(wl0y - ay, ay - wh0y));
-            const float ez = fmaxf(0.f, fmaxf(wl0z - az, az - wh0z));
-            const float dmin2 = ex * ex + ey * ey + ez * ez;
-            const float fx = fmaxf(fabsf(ax - wl0x), fabsf(ax - wh0x));
-            const float fy = fmaxf(fabsf(ay - wl0y), fabsf(ay - wh0y));
-            const float fz = fmaxf(fabsf(az - wl0z), fabsf(az - wh0z));
-            const float dmax2 = fx * fx + fy * fy + fz * fz;
-            in = dmax2 < cc.rin2;
-            sh = !in && dmin2 < cc.rout2;
-            nr = kNear && dmin2 < rnear2;
-        }
-        const unsigned short off = (unsigned short)(c * (int)sizeof(Cand));
-        if (kNear) {
-            // near atoms inside the cutoff for every point of the warp go to the
-            // front of wn, near atoms crossing it (large warp boxes) to the back;
-            // past kNearCap entries they stay on the FP32 lists
-            const bool ni = nr && in, ns = nr && sh;
-            const unsigned bni = __ballot_sync(0xffffffffu, ni);
-            const unsigned bns = __ballot_sync(0xffffffffu, ns);
-            const int room = kNearCap - n_ni - n_ns;
-            const int ti = min(__popc(bni), room);
-            const int ts = min(__popc(bns), room - ti);
-            const int ai = __popc(bni & lt), as = __popc(bns & lt);
-            if (ni && ai < ti) {
-                wn[n_ni + ai] = off;
-                in = false;
+    // groups of 32 per turn: two in split bricks, whose few warps wait for the
+    // ballots of one group with the boxes of the other (32^3 grid 36.9 -> 34.9 us);
+    // elsewhere other warps fill the wait and the second group only takes registers
+    constexpr int kGroups = P == 1 ? 2 : 1;
+    for (int base = 0; base < n_cand; base += 32 * kGroups) {
+        bool in[kGroups], sh[kGroups], nr[kGroups];
+#pragma unroll
+        for (int h = 0; h < kGroups; ++h) {
+            const int c = base + 32 * h + lane;
+            in[h] = sh[h] = nr[h] = false;
+            if (c < n_cand) {
+                const float4 a = *reinterpret_cast<const float4*>(&s.cand[c].ax);
+                const float ax = a.x, ay = a.z, az = a.w;
+                const float ex = fmaxf(0.f, fmaxf(wl0x - ax, ax - wh0x));
+                const float ey = fmaxf(0.f, fmaxf(wl0y - ay, ay - wh0y));
+                const float ez = fmaxf(0.f, fmaxf(wl0z - az, az - wh0z));
+                const float dmin2 = ex * ex + ey * ey + ez * ez;
+                const float fx = fmaxf(fabsf(ax - wl0x), fabsf(ax - wh0x));
+                const float fy = fmaxf(fabsf(ay - wl0y), fabsf(ay - wh0y));
+                const float fz = fmaxf(fabsf(az - wl0z), fabsf(az - wh0z));
+                const float dmax2 = fx * fx + fy * fy + fz * fz;
+                in[h] = dmax2 < cc.rin2;
+                sh[h] = !in[h] && dmin2 < cc.rout2;
+                nr[h] = kNear && dmin2 < rnear2;
             }
-            if (ns && as < ts) {
-                wn[kNearCap - 1 - (n_ns + as)] = off;
-                sh = false;
-            }
-            n_ni += ti;
-            n_ns += ts;
         }
-        const unsigned bi = __ballot_sync(0xffffffffu, in);
-        const unsigned bs = __ballot_sync(0xffffffffu, sh);
-        if (in) wl[n_in + __popc(bi & lt)] = off;
-        if (sh) wl[kMaxCand - 1 - (n_sh + __popc(bs & lt))] = off;
-        n_in += __popc(bi);
-        n_sh += __popc(bs);
+#pragma unroll
+        for (int h = 0; h < kGroups; ++h) {
+            const unsigned short off =
+                (unsigned short)((base + 32 * h + lane) * (int)sizeof(Cand));
+            if (kNear) {
+                // near atoms inside the cutoff for every point of the warp go to the
+                // front of wn, near atoms crossing it (large warp boxes) to the back;
+                // past kNearCap entries they stay on the FP32 lists
+                const bool ni = nr[h] && in[h], ns = nr[h] && sh[h];
+                const unsigned bni = __ballot_sync(0xffffffffu, ni);
+                const unsigned bns = __ballot_sync(0xffffffffu, ns);
+                const int room = kNearCap - n_ni - n_ns;
+                const int ti = min(__popc(bni), room);
+                const int ts = min(__popc(bns), room - ti);
+                const int ai = __popc(bni & lt), as = __popc(bns & lt);
+                if (ni && ai < ti) {
+                    wn[n_ni + ai] = off;
+                    in[h] = false;
+                }
+                if (ns && as < ts) {
+                    wn[kNearCap - 1 - (n_ns + as)] = off;
+                    sh[h] = false;
+                }
+                n_ni += ti;
+                n_ns += ts;
+            }
+            const unsigned bi = __ballot_sync(0xffffffffu, in[h]);
+            const unsigned bs = __ballot_sync(0xffffffffu, sh[h]);
+            if (in[h]) wl[n_in + __popc(bi & lt)] = off;
+            if (sh[h]) wl[kMaxCand - 1 - (n_sh + __popc(bs & lt))] = off;
+            n_in += __popc(bi);
+            n_sh += __popc(bs);
+        }
     }
     __syncwarp();
 

@@ -701,85 +701,107 @@ __device__ __forceinline__ void acc_cart(const double* t, double xf, double yf, 
     z = __dadd_rn(__dadd_rn(__dmul_rn(t[6], xf), __dmul_rn(t[7], yf)), __dmul_rn(t[8], zf));
 }
 
-// Marks the points that one atom image covers: block (x, y, z) takes image y
-// of atom x, and blocks z share its box. An image covers points whose
-// fractional distance along axis d is at most sigma / width_d, so only the
-// lattice box of that half-width (a thousandth of a spacing wider, far above
-// the rounding of its FP64 bounds) is tested, with the reference's own
-// expressions; the other points cannot pass the test. Every covered point is
-// written by whichever images cover it, all with the same 0. Testing every
-// point against every image took 2.3 ms on a 65 x 63 x 64 grid of a 424-atom
-// cell, 3e9 tests; this makes 2.4e6 in 23 us, most of it the turnover of blocks
-// whose image misses the cell and that end at once (32 us with 256 threads a
-// block; 46 us with a loop over the 27 images in one block, where each miss
-// costs the block its latency).
+// Marks the points that an atom's images cover; blocks y share the atom's boxes.
+// An image covers points whose fractional distance along axis d is at most
+// sigma / width_d, so only the lattice box of that half-width (a thousandth of a
+// spacing wider, far above the rounding of its FP64 bounds) is tested, with the
+// reference's own expressions; the other points cannot pass the test. Every
+// covered point is written by whichever images cover it, all with the same 0.
+// The lanes of a warp form the boxes of the 27 images at once, and the few that
+// reach the cell are then taken in turn. Testing every point against every image
+// took 2.3 ms on a 65 x 63 x 64 grid of a 424-atom cell, 3e9 tests; this makes
+// 2.4e6 in 17 us (a block per image, most of which miss the cell, 23 us; a loop
+// over the 27 images in one block, where each miss costs its latency, 46 us).
 constexpr int kAccAxis = 1024;  // axis values held on chip (longer boxes divide per point)
 constexpr int kAccThreads = 128;
 
-__global__ void __launch_bounds__(kAccThreads) acc_mark_kernel(const double4* __restrict__ atoms,
-                                                       const __grid_constant__ AccParams P,
-                                                       uint8_t* __restrict__ out) {
-    __shared__ double axis[kAccAxis];
-    const double4 at = atoms[blockIdx.x];
-    const double s = sqrt(at.w);
-    if (!(s > 0.0)) return;  // r^2 < 0 holds nowhere
-    const int m = blockIdx.y;
+__device__ __forceinline__ void mark_image(const AccParams& P, const double4& at, int m,
+                                           const int* l, const int* n, double* axis,
+                                           uint8_t* __restrict__ out) {
     const double q[3] = {__dadd_rn(at.x, (double)(m / 9 - 1)),
                          __dadd_rn(at.y, (double)((m / 3) % 3 - 1)),
                          __dadd_rn(at.z, (double)(m % 3 - 1))};
-    int lo[3], len[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double nm1 = (double)(P.n[d] - 1), w = s * P.reach[d];
-        const double a = fmax(ceil((q[d] - w) * nm1 - 1e-3), 0.0);
-        const double b = fmin(floor((q[d] + w) * nm1 + 1e-3), nm1);
-        if (!(a <= b)) return;  // the same for the whole block
-        lo[d] = (int)a;
-        len[d] = (int)b - (int)a + 1;
-    }
     double ix, iy, iz;
     acc_cart(P.t, q[0], q[1], q[2], ix, iy, iz);  // src/computegridsheet.h:134-140
-    const bool table = (int64_t)len[0] + len[1] + len[2] <= kAccAxis;
+    const bool table = (int64_t)n[0] + n[1] + n[2] <= kAccAxis;
     if (table) {
-        for (int e = threadIdx.x; e < len[0] + len[1] + len[2]; e += blockDim.x) {
-            const int d = e < len[0] ? 0 : e < len[0] + len[1] ? 1 : 2;
-            const int k = e - (d > 0 ? len[0] : 0) - (d > 1 ? len[1] : 0);
-            axis[e] = __ddiv_rn((double)(lo[d] + k), (double)(P.n[d] - 1));
+        __syncthreads();  // the table of the image before is no longer read
+        for (int e = threadIdx.x; e < n[0] + n[1] + n[2]; e += blockDim.x) {
+            const int d = e < n[0] ? 0 : e < n[0] + n[1] ? 1 : 2;
+            const int k = e - (d > 0 ? n[0] : 0) - (d > 1 ? n[1] : 0);
+            axis[e] = __ddiv_rn((double)(l[d] + k), (double)(P.n[d] - 1));
         }
         __syncthreads();
     }
-    const int64_t total = (int64_t)len[0] * len[1] * len[2];
-    for (int64_t c = blockIdx.z * (int64_t)blockDim.x + threadIdx.x; c < total;
-         c += (int64_t)gridDim.z * blockDim.x) {
+    const int64_t total = (int64_t)n[0] * n[1] * n[2];
+    for (int64_t c = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; c < total;
+         c += (int64_t)gridDim.y * blockDim.x) {
         int i, j, k;
         if (total <= INT32_MAX) {
-            const unsigned u = (unsigned)c, row = u / (unsigned)len[2];
-            k = (int)(u - row * (unsigned)len[2]);
-            i = (int)(row / (unsigned)len[1]);
-            j = (int)(row - (unsigned)i * (unsigned)len[1]);
+            const unsigned u = (unsigned)c, row = u / (unsigned)n[2];
+            k = (int)(u - row * (unsigned)n[2]);
+            i = (int)(row / (unsigned)n[1]);
+            j = (int)(row - (unsigned)i * (unsigned)n[1]);
         } else {
-            const int64_t row = c / len[2];
-            k = (int)(c - row * len[2]);
-            i = (int)(row / len[1]);
-            j = (int)(row - (int64_t)i * len[1]);
+            const int64_t row = c / n[2];
+            k = (int)(c - row * n[2]);
+            i = (int)(row / n[1]);
+            j = (int)(row - (int64_t)i * n[1]);
         }
         double xf, yf, zf, x, y, z;
         if (table) {
             xf = axis[i];
-            yf = axis[len[0] + j];
-            zf = axis[len[0] + len[1] + k];
+            yf = axis[n[0] + j];
+            zf = axis[n[0] + n[1] + k];
         } else {
-            xf = __ddiv_rn((double)(lo[0] + i), (double)(P.n[0] - 1));
-            yf = __ddiv_rn((double)(lo[1] + j), (double)(P.n[1] - 1));
-            zf = __ddiv_rn((double)(lo[2] + k), (double)(P.n[2] - 1));
+            xf = __ddiv_rn((double)(l[0] + i), (double)(P.n[0] - 1));
+            yf = __ddiv_rn((double)(l[1] + j), (double)(P.n[1] - 1));
+            zf = __ddiv_rn((double)(l[2] + k), (double)(P.n[2] - 1));
         }
         acc_cart(P.t, xf, yf, zf, x, y, z);
         const double dx = __dsub_rn(x, ix), dy = __dsub_rn(y, iy), dz = __dsub_rn(z, iz);
         const double r2 =
             __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
         if (r2 < at.w)  // src/computegridsheet.h:148
-            out[(size_t)(lo[2] + k) + (size_t)(lo[1] + j) * P.n[2] +
-                (size_t)(lo[0] + i) * P.n[1] * P.n[2]] = 0;
+            out[(size_t)(l[2] + k) + (size_t)(l[1] + j) * P.n[2] +
+                (size_t)(l[0] + i) * P.n[1] * P.n[2]] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(kAccThreads)
+    acc_mark_kernel(const double4* __restrict__ atoms, const __grid_constant__ AccParams P,
+                    uint8_t* __restrict__ out) {
+    __shared__ double axis[kAccAxis];
+    const double4 at = atoms[blockIdx.x];
+    const double s = sqrt(at.w);
+    if (!(s > 0.0)) return;  // r^2 < 0 holds nowhere
+    const int lane = threadIdx.x & 31;
+    int lo[3] = {0, 0, 0}, len[3] = {0, 0, 0};  // of image `lane`
+    bool any = lane < 27;
+    if (any) {
+        const double q[3] = {__dadd_rn(at.x, (double)(lane / 9 - 1)),
+                             __dadd_rn(at.y, (double)((lane / 3) % 3 - 1)),
+                             __dadd_rn(at.z, (double)(lane % 3 - 1))};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double nm1 = (double)(P.n[d] - 1), w = s * P.reach[d];
+            const double a = fmax(ceil((q[d] - w) * nm1 - 1e-3), 0.0);
+            const double b = fmin(floor((q[d] + w) * nm1 + 1e-3), nm1);
+            any = any && a <= b;
+            lo[d] = any ? (int)a : 0;
+            len[d] = any ? (int)b - (int)a + 1 : 0;
+        }
+    }
+    // the same in every warp of the block
+    for (unsigned left = __ballot_sync(0xffffffffu, any); left; left &= left - 1) {
+        const int m = __ffs(left) - 1;
+        int l[3], n[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            l[d] = __shfl_sync(0xffffffffu, lo[d], m);
+            n[d] = __shfl_sync(0xffffffffu, len[d], m);
+        }
+        mark_image(P, at, m, l, n, axis, out);
     }
 }
 
@@ -804,11 +826,10 @@ extern "C" int er_accessibility(er_ctx* ctx, int fw_id, int nx, int ny, int nz, 
     P.n[0] = nx; P.n[1] = ny; P.n[2] = nz;
     ER_CUDA(ctx, cudaMemsetAsync(mask, 1, (size_t)n, st));
     if (f->n_atoms > 0) {
-        // few atoms share each box among more blocks
+        // sixteen blocks per SM: few atoms share their boxes among more blocks
         const unsigned parts =
-            (unsigned)std::max(1, std::min(64, 4 * ctx->num_sms / f->n_atoms));
-        er::acc_mark_kernel<<<dim3((unsigned)f->n_atoms, 27, parts), er::kAccThreads, 0,
-                              st>>>(
+            (unsigned)std::max(1, std::min(64, 16 * ctx->num_sms / f->n_atoms));
+        er::acc_mark_kernel<<<dim3((unsigned)f->n_atoms, parts), er::kAccThreads, 0, st>>>(
             f->dev.atom_frac, P, mask);
         ER_CUDA(ctx, cudaGetLastError());
     }

@@ -15,8 +15,10 @@
 //    to the box centre, so FP32 never holds magnitudes above rc + box.
 //  * Candidate atom images come from the framework's cell list: one contiguous
 //    image range per (y, z) row of cells, with the x range of each row pruned
-//    by the cutoff circle. Passing candidates are compacted in order (block
-//    scans, so the order is deterministic) into shared memory.
+//    by the cutoff circle. Passing candidates are compacted in order (ballots
+//    and prefix sums, so the order is deterministic) into shared memory.
+//  * Atoms far from a fine grid's brick and inside the cutoff of all of it are
+//    summed at fewer nodes and interpolated to its points (far_field).
 //  * Each warp splits the CTA candidates against its own box into an inner
 //    list (inside the cutoff for every point of the warp: no test needed) and
 //    a shell list (cutoff tested per pair). Lists are u16 byte offsets.
@@ -28,7 +30,7 @@
 //  * Shell pairs whose FP32 r^2 lies within a proven error window of rc^2 are
 //    re-decided in FP64 with the reference's own expression order, so the set
 //    of summed pairs equals the FP64 reference's set exactly.
-//  * Accumulation: FP32 over chunks of 64 atoms, chunk sums added into FP64
+//  * Accumulation: FP32 over chunks of 8 to 64 atoms, chunk sums added into FP64
 //    per-point totals (ER_PREC_COMP, ER_PREC_NEAR64), or FP32 over the whole
 //    list (ER_PREC_FP32). ER_PREC_NEAR64 (the default) evaluates the pairs of
 //    atoms within kNearR of a warp's points in FP64: those large terms carry

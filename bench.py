@@ -3,7 +3,7 @@
 Workload (one "step"): grids of 256 seeded triclinic frameworks (a, b, c in
 [8, 40] A, angles in [60, 120] deg, 100-5000 atoms log-uniform capped at 0.16
 atoms/A^3, 8 atom types, probes CH4 / Xe / Kr, grid spacing 0.1-0.2 A, cutoff
-12.5 A) computed by one persistent launch over a device work queue replayed
+12.5 A) computed by one launch over a device work queue replayed
 as a CUDA graph, in the default precision mode (ER_PREC_NEAR64: FP32 pair
 terms, pairs of atoms within 5 A of a warp's points in FP64; within 1e-5
 relative of FP64 on E < -10 K points). Data are synthetic (no dataset ships
@@ -337,7 +337,7 @@ def run_ours(args, ws, rank, local, pg):
     points_step = float(sum(int(np.prod(f.dims)) for f in fws))
     outs = [torch.empty(f.dims, dtype=torch.float32, device="cuda") for f in fws]
     jobs = [(u, f.dims, o.data_ptr()) for u, f, o in zip(ups, fws, outs)]
-    # one persistent launch in the default (NEAR64) mode; the kernel variant of
+    # one launch in the default (NEAR64) mode; the kernel variant of
     # each job class picked by the autotuner at plan creation, outside the timing
     plan = ctx.batch_plan(jobs, er.ER_BATCH_PERSISTENT | er.ER_BATCH_AUTOTUNE)
     tiles = [plan.tile(k) for k in range(len(jobs))]
@@ -409,7 +409,7 @@ def run_ours(args, ws, rank, local, pg):
             e2e_times.append(dt)
     t_e2e = max_over_ranks(sum(e2e_times) / len(e2e_times), pg)
 
-    # roofline of the dominant (persistent) kernel
+    # roofline of the dominant (batch) kernel
     t_kernel = sum(times) / len(times)
     achieved = pairs_step * PAIR_INSTR / t_kernel
     roof = {"bound": "fp32", "achieved": achieved / 1e12, "peak": fp32_rate / 1e12,
@@ -481,7 +481,7 @@ def run_ours(args, ws, rank, local, pg):
 def run_batch_small(ctx, fws, l2buf, fp32_rate, dims=(32, 32, 32)):
     """Many small jobs, where one launch per job leaves the GPU idle: the 256
     batch frameworks each on a 32^3 grid (the config-1 grid size: 16-32
-    bricks per job against 444 resident CTA slots), one persistent launch
+    bricks per job against 444 resident CTA slots), one batched launch
     against one plain launch per job (both graph-replayed, default mode)."""
     import torch
 
@@ -825,7 +825,7 @@ def run_serving(ctx, args):
 
 
 def load_traffic(points_step):
-    """DRAM bytes per launch of the persistent kernel from the committed ncu
+    """DRAM bytes per launch of the batch kernel from the committed ncu
     capture of a smaller batch (profiles/grid_persistent_traffic.json), scaled
     to this launch by grid points (the traffic is the grid store)."""
     p = os.path.join(ROOT, "profiles", "grid_persistent_traffic.json")

@@ -19,9 +19,9 @@
 //                offsets (a cycle with non-zero net translation, self-links
 //                included) -- the same verdict as the reference's DFS, which
 //                checks every link of the component against a spanning walk
-//   5. block     channel roots are marked in the label array; every point
-//                walks to its root: pocket points -> 1e13 (host double grid)
-//                or mask = 1 (device), and the pocket roots are counted
+//   5. block     every point walks to its root and meets a channel's or not:
+//                pocket points -> 1e13 (host double grid) or mask = 1 (device),
+//                and the pocket roots are counted
 // The reference numbers segments in the order its flood fill meets them, by
 // smallest index: roots ranked in index order (compress and number), needed
 // only when the caller asks for the numbers.
@@ -392,6 +392,15 @@ __global__ void __launch_bounds__(256) cc_face_links(const int* __restrict__ lab
     }
 }
 
+// The channel roots, by value where they are few (a grid's channels usually are
+// one or two): copying them up and marking their labels took 2 of 75 us of a 64^3
+// mask's call.
+// Otherwise n is 0 and the roots are marked.
+struct Channels {
+    int n = 0;
+    int root[16];
+};
+
 // Channel roots r become -2 - r: the walk to a root ends at any negative label.
 __global__ void cc_mark_channels(const int* __restrict__ roots, int n, int* __restrict__ lab) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -403,17 +412,20 @@ __global__ void cc_mark_channels(const int* __restrict__ roots, int n, int* __re
 // the pockets (roots that no channel marking reached).
 template <bool MASK>
 __global__ void __launch_bounds__(256) cc_block(const int* __restrict__ lab, int64_t n,
+                                                const __grid_constant__ Channels ch,
                                                 double* __restrict__ E,
                                                 uint8_t* __restrict__ mask, PocketCounters* cnt) {
     int roots = 0;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
          p += (int64_t)gridDim.x * blockDim.x) {
         int x = (int)p, l = lab[p];
-        roots += l == x;
         while (l >= 0 && l != x) {
             x = l;
             l = lab[x];
         }
+        for (int k = 0; k < ch.n; ++k)
+            if (l == ch.root[k]) l = -1;
+        roots += l == (int)p;
         if (MASK) mask[p] = l >= 0;
         else if (l >= 0) E[p] = 1e13;
     }
@@ -508,12 +520,12 @@ struct LinkLayout {
 // Links copied back with their count, before it is known (the others follow).
 constexpr int64_t kFirstLinks = 2048;
 
-// Labels the grid E (device), finds the channels and marks their roots in
-// ps.lab, on stream st, which it synchronises once (twice past kFirstLinks
-// links). With `numbers` the segment of every point goes to ps.seg.
+// Labels the grid E (device) and finds the channels, whose roots go to ch or are
+// marked in ps.lab, on stream st, which it synchronises once (twice past
+// kFirstLinks links). With `numbers` the segment of every point goes to ps.seg.
 template <typename G>
 static int label_and_classify(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, const G* E,
-                              double thr, int nx, int ny, int nz, bool numbers) {
+                              double thr, int nx, int ny, int nz, bool numbers, Channels& ch) {
     const int64_t n = (int64_t)nx * ny * nz;
     const LinkLayout L(nx, ny, nz);
     const int64_t tiles = (int64_t)((nz + kTK - 1) / kTK) * ((ny + kTJ - 1) / kTJ) *
@@ -566,7 +578,10 @@ static int label_and_classify(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, c
     // a fixed order makes the host pass independent of the insertion order
     std::sort(links.begin(), links.end());
     const std::vector<int> channels = channel_roots(links);
-    if (!channels.empty()) {
+    if (channels.size() <= sizeof(ch.root) / sizeof(int)) {
+        ch.n = (int)channels.size();
+        std::copy(channels.begin(), channels.end(), ch.root);
+    } else {
         const size_t bytes = channels.size() * sizeof(int);
         if (ps.host.ensure(bytes) != ER_OK || ps.flags.ensure_on(bytes, ctx->pool, st) != ER_OK)
             return set_error(ctx, ER_ERR_NOMEM, "pockets: channel list allocation");
@@ -626,12 +641,13 @@ extern "C" int er_block_pockets(er_ctx* ctx, double* grid, int nx, int ny, int n
         return set_error(ctx, ER_ERR_NOMEM, "pockets: grid allocation failed");
     double* dE = (double*)ps.mask.ptr;
     ER_CUDA(ctx, cudaMemcpyAsync(dE, grid, n * sizeof(double), cudaMemcpyHostToDevice, st));
+    Channels ch;
     if ((stt = label_and_classify(ctx, ps, st, dE, 15.0 * temperature, nx, ny, nz,
-                                  segments_out != nullptr)) != ER_OK)
+                                  segments_out != nullptr, ch)) != ER_OK)
         return stt;
     PocketCounters* cnt = (PocketCounters*)ps.misc.ptr;
-    cc_block<false><<<block_grid(ctx, n), 256, 0, st>>>((const int*)ps.lab.ptr, n, dE, nullptr,
-                                                        cnt);
+    cc_block<false><<<block_grid(ctx, n), 256, 0, st>>>((const int*)ps.lab.ptr, n, ch, dE,
+                                                        nullptr, cnt);
     ER_CUDA(ctx, cudaGetLastError());
     int np = 0;
     ER_CUDA(ctx, cudaMemcpyAsync(&np, &cnt->pockets, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -654,12 +670,13 @@ int block_pockets_device_on(er_ctx* ctx, PocketScratch& ps, cudaStream_t st, con
     if (stt != ER_OK) return stt;
     const int64_t n = (int64_t)nx * ny * nz;
     if ((stt = ensure_pocket_scratch(ctx, ps, st, nx, ny, nz, false)) != ER_OK) return stt;
-    if ((stt = label_and_classify(ctx, ps, st, grid, 15.0 * temperature, nx, ny, nz, false)) !=
+    Channels ch;
+    if ((stt = label_and_classify(ctx, ps, st, grid, 15.0 * temperature, nx, ny, nz, false, ch)) !=
         ER_OK)
         return stt;
     PocketCounters* cnt = (PocketCounters*)ps.misc.ptr;
-    cc_block<true><<<block_grid(ctx, n), 256, 0, st>>>((const int*)ps.lab.ptr, n, nullptr, mask_out,
-                                                       cnt);
+    cc_block<true><<<block_grid(ctx, n), 256, 0, st>>>((const int*)ps.lab.ptr, n, ch, nullptr,
+                                                       mask_out, cnt);
     ER_CUDA(ctx, cudaGetLastError());
     int np = 0;
     ER_CUDA(ctx, cudaMemcpyAsync(&np, &cnt->pockets, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -28,3 +28,20 @@ def test_widom_layout_paths(ctx, n, masked):
     o = sums(P, f.t_matrix, f.rep, f.rc2, T, 77, n, mask=mask)
     assert r["n_blocked"] == o["n_blocked"] and r["n_insertions"] == n
     assert abs(r["sum_w"] - o["sum_w"]) <= 1e-6 * o["sum_w"]
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (2, 3, 32), (3, 2, 33), (4, 5, 34), (3, 4, 64), (5, 3, 65),
+                                  (2, 2, 66), (65, 33, 2), (40, 2, 97)])
+def test_widom_mask_rows(ctx, dims):
+    """Mask rows around the 32 cells that a warp takes at a time, and its last
+    grid point blocked: the same insertions are blocked as in the oracle."""
+    f = synth.config1(12)
+    P = f.particles()
+    fw = ctx.upload(P, f.t_matrix, f.rep, f.rc2)
+    mask = (np.random.default_rng(dims[2]).random(dims) < 0.03).astype(np.uint8)
+    mask[-1, -1, -1] = 1
+    r = ctx.henry(fw, T, 4096, seed=78, block_mask=mask, want_energies=True)
+    fw.release()
+    o = oracle.henry(P, f.t_matrix, f.rep, f.rc2, T, 78, 4096, mask=mask, want_energies=True)
+    assert r["n_blocked"] == o["n_blocked"] > 0
+    assert np.array_equal(np.isinf(r["energies"]), np.isinf(o["energies"]))

@@ -238,16 +238,22 @@ int check_grid_dims(er_ctx* ctx, int nx, int ny, int nz, const char* who) {
 
 // Squared distance from which on a P = 8 brick's atoms are interpolated (0: no
 // atom is). h = the larger spacing of the two interpolated axes. 46 h bounds the
-// interpolation error of the smooth attraction; 4 A + 16 h that of the steep
-// terms near 5 A, where 46 h alone is not far enough (h < 0.13 A: 2.7e-5 K root
-// mean square at 5.0 A and h = 0.1 A, 3e-6 K at 5.6 A); the near pairs' 5 A stay
-// outside. Grids coarser than about 0.2 A have no atom that far from a brick and
+// interpolation error of the smooth attraction; max(4 A, sigma) + 16 h that of the
+// steep terms, where 46 h alone is not far enough (h < 0.13 A: at sigma 3.5 A 2.7e-5
+// K root mean square at 5.0 A and h = 0.1 A, 3e-6 K at 5.6 A). Their error grows as
+// sigma^12, so sigma is the framework's largest mixed one: with 4 A in its place the
+// error of the |E| < 1e3 K points of a pore cell at h = 0.12 A was 4.1e-4 K root mean
+// square at sigma 5 A, 2.9e-3 at 6 and 4.7e-2 at 8, against 1.7e-4, 8.5e-4 and 4.7e-3
+// of the FP32 terms alone; this way the interpolation's own part stays at or below
+// 2.2e-5 K (epsilon 94 K, 0.08 atoms / A^3, sigma up to 8 A, h 0.03 to 0.18 A). The
+// near pairs' 5 A stay outside. Grids coarser than about 0.2 A have no atom that far from a brick and
 // inside the cutoff of all its points.
 static float far_distance2(const FwRecord& fw, const GridTask& t, double* diag = nullptr) {
     if (t.tile_p != 8) return 0.f;
     const double ha = fw.cell_len[0] / (t.nx - 1), hc = fw.cell_len[2] / (t.nz - 1);
     const double hm = std::max(ha, hc);
-    const double rf = std::max({(double)kNearR, 4.0 + 16.0 * hm, 46.0 * hm});
+    const double rf =
+        std::max({(double)kNearR, std::max(4.0, fw.sig_max) + 16.0 * hm, 46.0 * hm});
     const double* r = fw.dev.r;
     double diag2 = 0.0;  // of the brick's Cartesian box
     for (int d = 0; d < 3; ++d) {
@@ -618,6 +624,7 @@ void fw_record(const HostFramework& hf, size_t n_img, const FwLayout& L, void* b
     rec.volume = fabs(hf.t[0] * (hf.t[4] * hf.t[8] - hf.t[5] * hf.t[7]) -
                       hf.t[1] * (hf.t[3] * hf.t[8] - hf.t[5] * hf.t[6]) +
                       hf.t[2] * (hf.t[3] * hf.t[7] - hf.t[4] * hf.t[6]));
+    rec.sig_max = hf.sig_max;
     rec.n_atoms = hf.n_atoms;
 }
 

@@ -25,6 +25,7 @@ struct FwRecord {
     double t[9] = {0};
     double cell_len[3] = {0, 0, 0};  // |a|, |b|, |c|
     double volume = 0.0;
+    double sig_max = 0.0;            // largest mixed sigma
     int n_atoms = 0;
 };
 

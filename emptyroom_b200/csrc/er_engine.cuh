@@ -1304,8 +1304,9 @@ __device__ __forceinline__ void fp64_lists(EngineSmem& s, const Pol& pol, const 
 // third axis, every lattice line along the second) instead of 2048 points, and
 // interpolated to the points in FP64. Rf (far_distance2) keeps the error of the
 // interpolation, which falls as (x + sqrt(x^2 + 1))^-8 with x = Rf over the
-// half-width 7.5 spacings, at a few 1e-6 K root mean square, below the rounding
-// of the FP32 pair terms; those are the same here as for the points. At 0.12 A
+// half-width 7.5 spacings and grows as sigma^12, below the rounding of the FP32
+// pair terms (1e-6 to 2e-5 K root mean square at epsilon 94 K, against 2e-5 to
+// 5e-3); those are the same here as for the points. At 0.12 A
 // about 60 % of a cell's pairs are far and cost a quarter: a 256^3 grid of 4096
 // atoms 8.70 -> 6.57 ms, 8 triclinic frameworks (54 M points) 16.76 -> 14.2 ms.
 constexpr int kFarN = 8;   // nodes per 16 lattice points

@@ -127,6 +127,7 @@ int prepare_framework(const er_framework_desc& d, double h, HostFramework& f, st
         if (c12f == 0.0f) c12f = 1.17549435e-38f;  // keep u3 * (C12 u3 - C6) NaN-free
         atom_par[2 * a] = c12f;
         atom_par[2 * a + 1] = -c6f;
+        f.sig_max = std::max(f.sig_max, sqrt(s2));
     }
     // Keep image a + n only if it can be within rc of the grid region
     // [0,1]^3: its fractional overshoot of slab d times the slab width w_d is a

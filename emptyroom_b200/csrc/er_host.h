@@ -21,6 +21,7 @@ struct HostFramework {
     double t[9] = {0};
     double r[9] = {0};                  // positioning frame (upper triangular)
     double rc2 = 0.0;
+    double sig_max = 0.0;               // largest mixed sigma of an atom with images
     double h = 2.0;
     int nc[3] = {1, 1, 1};
     double cell_lo[3] = {0, 0, 0};

@@ -42,3 +42,40 @@ def test_far_field_against_fp64(ctx, abc, angles, n, dims):
     assert np.array_equal(ctx.grid(fw, dims), same)
     plan.close()
     fw.release()
+
+
+def _pore(sigma, edge, seed, density=0.08):
+    """A wall of atoms of one mixed sigma around an empty sphere that the probe fits into."""
+    f = np.random.default_rng(seed).random((int(density * edge ** 3), 3))
+    return f[np.linalg.norm((f - 0.5) * edge, axis=1) > sigma + 3.2]
+
+
+@pytest.mark.parametrize("sigma, spacing", [(5.0, 0.12), (5.0, 0.10), (6.0, 0.12), (8.0, 0.15)])
+def test_far_field_of_large_sigma(ctx, sigma, spacing):
+    """Bulky probes: the steep terms reach further, and so must the atoms summed one by
+    one. Every other point of the grid is a point of the grid of twice the spacing,
+    which is too coarse for a far field: what its energies are off by is the rounding
+    of the FP32 terms, somewhat less of it (its larger warp boxes take more atoms to
+    FP64: a factor of 1.7 between 0.07 and 0.18 A). The interpolation may not add to
+    that: root mean square error at most twice the coarse grid's."""
+    import torch
+    edge = 2.0 * (sigma + 3.2) + 4.0
+    frac = _pore(sigma, edge, int(100 * sigma))
+    m = int(edge / spacing / 2) + 1
+    t = np.diag([edge] * 3)
+    fw = ctx.upload(er.particles(frac, np.full(len(frac), 94.0), np.full(len(frac), sigma * sigma)),
+                    t, er.replication_factors(t, 12.5), 12.5 ** 2)
+    rms, ok = [], None
+    for n in (m, 2 * m - 1):
+        e = torch.empty((n,) * 3, dtype=torch.float32, device="cuda")
+        ref = torch.empty((n,) * 3, dtype=torch.float64, device="cuda")
+        ctx.grid_device(fw, (n,) * 3, e.data_ptr())
+        ctx.grid_device(fw, (n,) * 3, ref.data_ptr(), precision=er.ER_PREC_FP64, f64=True)
+        ctx.synchronize()
+        step = 1 if n == m else 2
+        e, ref = (x[::step, ::step, ::step] for x in (e, ref))
+        ok = ref.abs() < 1e3 if ok is None else ok
+        rms.append(float((e.double() - ref)[ok].pow(2).mean().sqrt()))
+    fw.release()
+    assert int(ok.sum()) > 500
+    assert rms[1] <= 2.0 * rms[0]

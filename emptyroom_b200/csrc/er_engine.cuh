@@ -85,9 +85,8 @@ struct PrecTraits {
 // lists: with 16 the mean error on E < -10 K points was within 3 % of the one
 // without a far field, either way; with 8 it is 4-10 % below it (five cells at
 // 0.1-0.155 A), for 2 % more time. And for Widom warps of 128 points, whose boxes
-// have fewer atoms within kNearR than those of 256: with 16 the mean error of 1.5e6
-// insertions was 12 % above that of 256-point warps, with 8 it is 3.5 % above it
-// and 2-4 % below it at 1.2e6, 2e5 and 32768.
+// have fewer atoms within kNearR than those of 256: with 8 the mean error of 2e5
+// and 32768 insertions is 2-4 % below the one with 16.
 constexpr int kShortChunk = 8;
 template <class Pol, int PREC>
 struct InnerChunk {

@@ -9,7 +9,7 @@
 //      position's point, then order the bins that straddle a warp boundary by
 //      insertion index (so every warp's point set, and with it every FP32
 //      rounding, is deterministic)
-//   5. energy  the shared LJ engine over 2048 (1024 for runs below 1.5 * 2^20)
+//   5. energy  the shared LJ engine over 2048 (1024 for runs below 1e6)
 //              points per CTA, in bin order
 //   6. reduce  FP64 log-sum-exp of exp(-E/T) and E exp(-E/T) in insertion
 //              order with a fixed tree: (m, s, se) with sum w = s e^m.
@@ -29,12 +29,16 @@ namespace er {
 // Insertions per thread of the energy kernel: 4 below kHenrySmallN, where a run
 // fills few waves of CTAs, whose more numerous and smaller halves finish sooner,
 // and where its points lie so far apart that a smaller CTA reaches fewer atoms;
-// 8 from there on, each atom loaded serving twice the points. Measured 8 / 4, us
-// a call: 1e6 insertions 297 / 275 (cell of 424 atoms), 835 / 698 (1500 atoms);
-// 2e6 433 / 448; 3e6 571 / 595; 1e7 1650 / 1800.
+// 8 from there on, each atom loaded serving twice the points. 4 is faster up to
+// 1.5e6 (8 / 4, us a call: 1e6 insertions 297 / 275 in a cell of 424 atoms, 835 /
+// 698 of 1500 atoms; 2e6 433 / 448; 1e7 1650 / 1800), but a warp of 128 points
+// takes fewer atoms to FP64 than one of 256, and from 1e6 on its energies are less
+// accurate: mean relative error on E < -10 K points, 1e6 insertions, 8 / 4: 3.84 /
+// 3.89e-8 (424 atoms, CH4), 4.62 / 4.82e-8 (424, Xe), 3.21 / 3.45e-8 (100, Kr),
+// 4.51 / 4.87e-8 (900, Kr).
 constexpr int kHenryP = 8;
 constexpr int kHenryPSmall = 4;
-constexpr int64_t kHenrySmallN = 3 << 19;
+constexpr int64_t kHenrySmallN = 1000000;
 inline int henry_points_per_thread(int64_t n) { return n < kHenrySmallN ? kHenryPSmall : kHenryP; }
 
 struct BinGeom {

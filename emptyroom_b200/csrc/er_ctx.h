@@ -201,6 +201,19 @@ int henry_reserve(er_ctx* ctx, HenryScratch& hs, int64_t n, cudaStream_t st);
 int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, uint64_t seed,
                   const uint8_t* block_mask, int mnx, int mny, int mnz, cudaStream_t st,
                   HenryScratch& hs, HenryOut* host_out);
+// Blocks of a Widom reduction of n energies (er_henry's and
+// er_henry_stats_noalloc's, so that both add in one order): four per SM, of at
+// least 2048 energies (fewer partial sums to merge), at most 4096. 64-bit, so that
+// no n below 2^31 overflows.
+struct ReduceBlocks {
+    int64_t chunk;  // energies per block
+    int blocks;
+    ReduceBlocks(const er_ctx* ctx, int64_t n) {
+        const int64_t most = std::min(4096, std::max(1, ctx->num_sms * 4));
+        chunk = std::max<int64_t>((n + most - 1) / most, 2048);
+        blocks = (int)((n + chunk - 1) / chunk);
+    }
+};
 void henry_finish(const HenryOut& h, int64_t n, double temperature, er_henry_result* out);
 // Pocket mask of an FP32 device grid (er_block_pockets_device) with scratch
 // `ps` on stream `st`; synchronises `st` (the segment classification runs on

@@ -696,12 +696,10 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
     else ER_CUDA(ctx, energy(henry_energy_kernel<kHenryPSmall, 1>, 1));
     ER_CUDA(ctx, cudaGetLastError());
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[3], st));
-    // at least 2048 insertions a block: fewer partial sums to merge
-    const int rblocks = std::min(4096, std::max(1, ctx->num_sms * 4));
-    const int chunk = std::max((n + rblocks - 1) / rblocks, 2048);
-    const int nrb = (n + chunk - 1) / chunk;
-    henry_reduce_kernel<<<nrb, 256, 0, st>>>(E, n, -1.0 / temperature, chunk, (Lse*)hs.part.ptr,
-                                             rdone, nblk, (HenryOut*)hs.res.ptr);
+    const ReduceBlocks rb(ctx, n);
+    henry_reduce_kernel<<<rb.blocks, 256, 0, st>>>(E, n, -1.0 / temperature, (int)rb.chunk,
+                                                   (Lse*)hs.part.ptr, rdone, nblk,
+                                                   (HenryOut*)hs.res.ptr);
     ER_CUDA(ctx, cudaGetLastError());
     if (hs.ev[0]) ER_CUDA(ctx, cudaEventRecord(hs.ev[4], st));
     if (host_out)

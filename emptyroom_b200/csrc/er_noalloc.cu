@@ -141,14 +141,10 @@ extern "C" int er_henry_stats_noalloc(er_ctx* ctx, const float* energies, int64_
     noalloc::Stats* scratch = nullptr;
     int st = noalloc::scratch_for(ctx, &scratch);
     if (st != ER_OK) return st;
-    // the block partition of er_henry's reduction of long runs (4 blocks per SM, at most
-    // kSlots), computed in 64-bit so that it cannot overflow at the top of the range
-    const int64_t rblocks = std::min<int64_t>(noalloc::kSlots, std::max(1, ctx->num_sms * 4));
-    const int64_t chunk = (n + rblocks - 1) / rblocks;
-    const int nrb = (int)((n + chunk - 1) / chunk);
-    noalloc::partial_kernel<<<nrb, 256, 0, ctx->stream>>>(energies, n, temperature, chunk,
-                                                           scratch);
-    noalloc::final_kernel<<<1, 256, 0, ctx->stream>>>(scratch, nrb);
+    const ReduceBlocks rb(ctx, n);  // er_henry's, at most kSlots
+    noalloc::partial_kernel<<<rb.blocks, 256, 0, ctx->stream>>>(energies, n, temperature, rb.chunk,
+                                                                 scratch);
+    noalloc::final_kernel<<<1, 256, 0, ctx->stream>>>(scratch, rb.blocks);
     ER_CUDA(ctx, cudaGetLastError());
     noalloc::Stats r;
     ER_CUDA(ctx, cudaMemcpyAsync(&r, scratch + noalloc::kSlots, sizeof(r), cudaMemcpyDeviceToHost,

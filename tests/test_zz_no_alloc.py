@@ -105,3 +105,19 @@ def test_noalloc_at_the_documented_maximum(ctx):
     finally:
         del E
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("n", [1, 2048, 2049, 37777, 200_000, 1_300_000])
+def test_noalloc_adds_in_er_henrys_order(ctx, n):
+    """The same blocks and the same trees: at T = 256 K, where E / T and E times
+    1 / T are the same number, every sum equals er_henry's bit for bit."""
+    import torch
+    f = synth.make_framework(42, (20.0, 19.0, 21.0), (80, 100, 95), 60, probe="Kr")
+    fw = ctx.upload(f.particles(), f.t_matrix, f.rep, f.rc2)
+    ref = ctx.henry(fw, 256.0, n, seed=8, want_energies=True)
+    fw.release()
+    E = torch.from_numpy(ref["energies"]).cuda()
+    st, got = _noalloc(ctx, E.data_ptr(), n, 256.0)
+    assert st == 0, _capi.lib().er_ctx_last_error(ctx.handle)
+    for key in ("log_scale", "sum_w_scaled", "sum_ew_scaled", "sum_w", "kh_mol_m3_pa"):
+        assert getattr(got, key) == ref[key], key

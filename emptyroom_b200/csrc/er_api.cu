@@ -366,19 +366,26 @@ int launch_grid_batch(er_ctx* ctx, const GridTask* d_tasks, const int* d_start, 
 // ------------------------------------------------------------------ autotuner
 // Picks the kernel variant (4 or 8 points per thread) for a class of jobs by
 // timing both, in the precision mode the jobs run in, on the same sample of
-// the job -- its first 16 x-layers, which are whole bricks for both variants
+// the job -- its first x-layers, which are whole bricks for both variants
 // -- and caches the faster one per class: (atoms per A^3 in half-octaves,
 // smallest grid spacing in quarter-octaves, cutoff in quarter-Angstroms,
-// precision mode).
+// precision mode, form). It times the kernels that the plan will launch: the
+// bricks of a batch in one launch (`one_launch`) are not divided among CTAs,
+// those of a launch of their own are where they are few. The form holds that
+// division and whether P = 8 has a far field.
 int tune_tile(er_ctx* ctx, const FwRecord& f, int nx, int ny, int nz, float* out, int prec,
-              int* tile_p) {
+              bool one_launch, int* tile_p) {
+    GridTask task[2];  // P = 4, P = 8
+    for (int v = 0; v < 2; ++v)
+        if (int st = fill_grid_task(ctx, f, nx, ny, nz, out, task[v], 4 << v)) return st;
     const double rho = (double)std::max(f.n_atoms, 1) / std::max(f.volume, 1e-9);
     double h = 1e30;
     const int dims[3] = {nx, ny, nz};
     for (int d = 0; d < 3; ++d) h = std::min(h, f.cell_len[d] / std::max(dims[d] - 1, 1));
-    const std::tuple<int, int, int, int> key((int)lround(2.0 * log2(rho)),
-                                             (int)lround(4.0 * log2(h)),
-                                             (int)lround(4.0 * sqrt(f.rc2)), prec);
+    const int split = one_launch ? 1 : grid_split(ctx, task_bricks(task[0]));
+    const std::tuple<int, int, int, int, int> key(
+        (int)lround(2.0 * log2(rho)), (int)lround(4.0 * log2(h)), (int)lround(4.0 * sqrt(f.rc2)),
+        prec, 2 * split + (task[1].far2 > 0.f ? 1 : 0));
     auto it = ctx->tune.find(key);
     if (it != ctx->tune.end()) {
         *tile_p = it->second;
@@ -390,21 +397,24 @@ int tune_tile(er_ctx* ctx, const FwRecord& f, int nx, int ny, int nz, float* out
     float best_ms = 0.f;
     int best = 4;
     // Both variants time the same first x-layers: a multiple of 16 large
-    // enough for four waves of the bigger (P = 8) bricks on this GPU, so
-    // neither variant is timed on an underfilled launch.
+    // enough for four waves of the bigger (P = 8) bricks on this GPU, so that
+    // neither is timed on an underfilled launch (a smaller grid is timed whole).
     const int nbyz = ((ny + 2 * kWJ - 1) / (2 * kWJ)) * ((nz + 2 * kWK - 1) / (2 * kWK));
     const int slots = 3 * ctx->num_sms;
     const int layers = 16 * std::max(1, (4 * slots + nbyz - 1) / nbyz);
     for (int P : {4, 8}) {
-        GridTask t;
-        int st = fill_grid_task(ctx, f, nx, ny, nz, out, t, P);
-        if (st != ER_OK) return st;
+        GridTask& t = task[P / 8];
         if (nx > layers) t.nb[0] = layers / (2 * P);
+        const int64_t bricks = task_bricks(t);
+        if (bricks > INT32_MAX) return set_error(ctx, ER_ERR_LIMIT, "grid: too many bricks");
         float ms_min = 1e30f;
         for (int rep = 0; rep < 3; ++rep) {
             ER_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
-            st = launch_grid_plain(ctx, t, prec);
-            if (st != ER_OK) return st;
+            if (P == 8) launch_variant<8, 1>(t, prec, (unsigned)bricks, ctx->stream);
+            else if (split == 4) launch_variant<4, 4>(t, prec, (unsigned)bricks, ctx->stream);
+            else if (split == 2) launch_variant<4, 2>(t, prec, (unsigned)bricks, ctx->stream);
+            else launch_variant<4, 1>(t, prec, (unsigned)bricks, ctx->stream);
+            ER_CUDA(ctx, cudaGetLastError());
             ER_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
             ER_CUDA(ctx, cudaEventSynchronize(e1));
             float ms = 0.f;
@@ -921,7 +931,7 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
         // (a far field needs P = 8 and always pays: nothing to time)
         if (autotune && dims_ok && tile_p == 4)
             st = tune_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device, prec,
-                           &tile_p);
+                           mode == ER_BATCH_PERSISTENT, &tile_p);
         GridTask t;
         if (st == ER_OK)
             st = fill_grid_task(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device, t,

@@ -109,7 +109,7 @@ struct er_ctx {
     std::map<int, er::FwRecord> fws;
     int next_fw = 1;
     double cell_edge = 2.0;  // cell-list edge (A)
-    std::map<std::tuple<int, int, int, int>, int> tune;  // autotuned kernel variant per job class
+    std::map<std::tuple<int, int, int, int, int>, int> tune;  // autotuned variant per job class
     // scratch
     er::DevBuf grid_f32;     // staging for host-bound grids
     er::DevBuf counter;      // scratch of the FP32 rate probe
@@ -186,7 +186,8 @@ CutoffConsts make_cutoff_consts(double rc2, double box_diag, double r2min);
 int check_grid_dims(er_ctx* ctx, int nx, int ny, int nz, const char* who);
 // Kernel variant (points per thread) of a grid where the caller asks for none:
 // the same for a single call, a batch, the server and a Widom batch, so that
-// their results are equal bit for bit.
+// their results are equal bit for bit. (A batch that the caller has autotuned
+// may take P = 8 where this says 4.)
 int default_tile(const er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, int prec);
 // Fills a grid task (validates dims) and launches the plain grid kernel on `st`.
 int fill_grid_task(er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, float* out,

@@ -28,3 +28,27 @@ def test_widom_warps_of_long_runs(ctx, n, points):
     names = [k for k in _kernels(ctx, lambda: ctx.henry(fw, 298.0, n, seed=1)) if "henry_energy" in k]
     fw.release()
     assert len(names) == 1 and f"henry_energy_kernel<{points}, 1>" in names[0]
+
+
+def _variants(names):
+    """(points per thread, CTAs per brick) of the grid kernels among `names`."""
+    return {tuple(int(x) for x in k.split("grid_kernel<")[1].split(">")[0].split(",")[1:])
+            for k in names if "grid_kernel<" in k}
+
+
+@pytest.mark.parametrize("n, split", [(32, 4), (50, 2), (80, 1)])
+def test_autotuner_times_what_the_plan_runs(n, split):
+    """A batch in one launch never divides its bricks, a launch of its own does where
+    they are few: the tuner times the one or the other."""
+    import torch
+    f = synth.config1(0)
+    out = torch.empty((n,) * 3, dtype=torch.float32, device="cuda")
+    for mode, division in ((er.ER_BATCH_PERSISTENT, 1), (er.ER_BATCH_PLAIN, split)):
+        with er.Context(0) as ctx:  # nothing tuned yet
+            fw = ctx.upload(f.particles(), f.t_matrix, f.rep, f.rc2)
+            plans = []
+            names = _kernels(ctx, lambda: plans.append(ctx.batch_plan(
+                [(fw, out.shape, out.data_ptr())], mode | er.ER_BATCH_AUTOTUNE | er.ER_BATCH_COMP)))
+            plans[0].close()
+            fw.release()
+        assert _variants(names) == {(4, division), (8, 1)}

@@ -635,6 +635,7 @@ void fw_record(const HostFramework& hf, size_t n_img, const FwLayout& L, void* b
                       hf.t[1] * (hf.t[3] * hf.t[8] - hf.t[5] * hf.t[6]) +
                       hf.t[2] * (hf.t[3] * hf.t[7] - hf.t[4] * hf.t[6]));
     rec.sig_max = hf.sig_max;
+    rec.sig_mean = hf.sig_mean;
     rec.n_atoms = hf.n_atoms;
 }
 

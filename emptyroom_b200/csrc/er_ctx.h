@@ -26,6 +26,7 @@ struct FwRecord {
     double cell_len[3] = {0, 0, 0};  // |a|, |b|, |c|
     double volume = 0.0;
     double sig_max = 0.0;            // largest mixed sigma
+    double sig_mean = 0.0;           // cube root of the mean sigma^3
     int n_atoms = 0;
 };
 

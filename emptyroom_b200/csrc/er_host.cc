@@ -105,7 +105,9 @@ int prepare_framework(const er_framework_desc& d, double h, HostFramework& f, st
         const double c6l = 4.0 * p.eps_with_adsorbate * s2 * s2 * s2;
         atom_lj64[2 * a] = c6l * s2 * s2 * s2;
         atom_lj64[2 * a + 1] = c6l;
+        f.sig_mean += s2 * sqrt(s2);
     }
+    f.sig_mean = cbrt(f.sig_mean / std::max(d.n_atoms, 1));
     for (int a = 0; a < d.n_atoms; ++a) {
         const er_particle& p = d.atoms[a];
         const double s2 = p.sig_with_adsorbate_squared;

@@ -22,6 +22,7 @@ struct HostFramework {
     double r[9] = {0};                  // positioning frame (upper triangular)
     double rc2 = 0.0;
     double sig_max = 0.0;               // largest mixed sigma of an atom with images
+    double sig_mean = 0.0;              // cube root of the atoms' mean sigma^3
     double h = 2.0;
     int nc[3] = {1, 1, 1};
     double cell_lo[3] = {0, 0, 0};

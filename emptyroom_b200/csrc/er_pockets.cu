@@ -822,6 +822,68 @@ __global__ void __launch_bounds__(kAccThreads)
     }
 }
 
+// The same from the points' side, for spheres that overlap many times over (below):
+// every point tests the images until one covers it.
+__global__ void acc_images_kernel(const double4* __restrict__ atoms, int n,
+                                  const __grid_constant__ AccParams P, double4* __restrict__ img) {
+    const int total = 27 * n;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
+        const int a = q / 27, m = q % 27;
+        const double4 at = atoms[a];
+        double x, y, z;
+        // src/computegridsheet.h:134-140
+        acc_cart(P.t, __dadd_rn(at.x, (double)(m / 9 - 1)),
+                 __dadd_rn(at.y, (double)((m / 3) % 3 - 1)), __dadd_rn(at.z, (double)(m % 3 - 1)),
+                 x, y, z);
+        img[q] = make_double4(x, y, z, at.w);
+    }
+}
+
+__global__ void __launch_bounds__(256)
+    acc_points_kernel(const double4* __restrict__ img, int nimg,
+                      const __grid_constant__ AccParams P, uint8_t* __restrict__ out) {
+    __shared__ double4 tile[512];
+    const int64_t n = (int64_t)P.n[0] * P.n[1] * P.n[2];
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    double x = 0, y = 0, z = 0;
+    bool open = p < n;
+    if (open) {
+        const int k = (int)(p % P.n[2]), j = (int)((p / P.n[2]) % P.n[1]),
+                  i = (int)(p / ((int64_t)P.n[1] * P.n[2]));
+        acc_cart(P.t, __ddiv_rn((double)i, (double)(P.n[0] - 1)),
+                 __ddiv_rn((double)j, (double)(P.n[1] - 1)),
+                 __ddiv_rn((double)k, (double)(P.n[2] - 1)), x, y, z);
+    }
+    for (int base = 0; base < nimg; base += 512) {
+        const int cnt = min(512, nimg - base);
+        if (!__syncthreads_or(open)) break;  // (also: the tile before is no longer read)
+        for (int q = threadIdx.x; q < cnt; q += blockDim.x) tile[q] = img[base + q];
+        __syncthreads();
+        for (int q = 0; open && q < cnt; ++q) {
+            const double4 w = tile[q];
+            const double dx = __dsub_rn(x, w.x), dy = __dsub_rn(y, w.y), dz = __dsub_rn(z, w.z);
+            const double r2 =
+                __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+            open = !(r2 < w.w);  // src/computegridsheet.h:148
+        }
+    }
+    if (p < n) out[p] = open ? 1 : 0;
+}
+
+// Marking takes c tests a point, c = the boxes that lie over it (27 images: at most
+// 3 along an axis); a point takes some multiple of 27 n / c images until one covers
+// it. So c^2 / n decides, at 18 (grids of few points, whose blocks are too few to
+// hide a point's chain of tests, 48). Measured boxes / points, us a call: 424 atoms
+// in 25.8 A, sigma 3.5 A (c^2 / n = 0.17), 65^3 71 / 1793; 259 in 12 A, 3.7 A (14),
+// 33^3 50 / 112, 65^3 130 / 197, 129^3 697 / 777; 150 in 10 A, 3.7 A (25) 51 / 76, 128
+// / 118, 709 / 480; 76 in 8 A, 3.7 A (48) 55 / 56, 133 / 85, 689 / 333; 76 in 8 A, 7 A
+// (2183) 131 / 34, 529 / 61, 3547 / 214.
+static bool acc_from_points(const FwRecord& f, const double* reach, int64_t points) {
+    double c = f.n_atoms;
+    for (int d = 0; d < 3; ++d) c *= std::min(2.0 * f.sig_mean * reach[d], 3.0);
+    return c * c > (points < 100000 ? 48.0 : 18.0) * f.n_atoms && f.n_atoms <= INT32_MAX / 27;
+}
+
 }  // namespace er
 
 extern "C" int er_accessibility(er_ctx* ctx, int fw_id, int nx, int ny, int nz, uint8_t* out) {
@@ -841,14 +903,25 @@ extern "C" int er_accessibility(er_ctx* ctx, int fw_id, int nx, int ny, int nz, 
     er::perpendicular_widths(f->t, w);
     for (int d = 0; d < 3; ++d) P.reach[d] = w[d] > 0.0 ? 1.0 / w[d] : INFINITY;
     P.n[0] = nx; P.n[1] = ny; P.n[2] = nz;
-    ER_CUDA(ctx, cudaMemsetAsync(mask, 1, (size_t)n, st));
-    if (f->n_atoms > 0) {
-        // sixteen blocks per SM: few atoms share their boxes among more blocks
-        const unsigned parts =
-            (unsigned)std::max(1, std::min(64, 16 * ctx->num_sms / f->n_atoms));
-        er::acc_mark_kernel<<<dim3((unsigned)f->n_atoms, parts), er::kAccThreads, 0, st>>>(
-            f->dev.atom_frac, P, mask);
+    if (er::acc_from_points(*f, P.reach, n)) {
+        const int nimg = 27 * f->n_atoms;
+        if (ctx->pocket.lab.ensure_on((size_t)nimg * sizeof(double4), ctx->pool, st))
+            return er::set_error(ctx, ER_ERR_NOMEM, "accessibility: scratch allocation failed");
+        double4* img = (double4*)ctx->pocket.lab.ptr;
+        er::acc_images_kernel<<<std::max(1, std::min((nimg + 255) / 256, ctx->num_sms * 8)), 256, 0,
+                                st>>>(f->dev.atom_frac, f->n_atoms, P, img);
+        er::acc_points_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(img, nimg, P, mask);
         ER_CUDA(ctx, cudaGetLastError());
+    } else {
+        ER_CUDA(ctx, cudaMemsetAsync(mask, 1, (size_t)n, st));
+        if (f->n_atoms > 0) {
+            // sixteen blocks per SM: few atoms share their boxes among more blocks
+            const unsigned parts =
+                (unsigned)std::max(1, std::min(64, 16 * ctx->num_sms / f->n_atoms));
+            er::acc_mark_kernel<<<dim3((unsigned)f->n_atoms, parts), er::kAccThreads, 0, st>>>(
+                f->dev.atom_frac, P, mask);
+            ER_CUDA(ctx, cudaGetLastError());
+        }
     }
     ER_CUDA(ctx, cudaMemcpyAsync(out, ctx->pocket.seg.ptr, (size_t)n, cudaMemcpyDeviceToHost, st));
     ER_CUDA(ctx, cudaStreamSynchronize(st));

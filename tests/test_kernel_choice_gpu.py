@@ -1,5 +1,6 @@
 """Which kernels a call launches, where the choice is the point: read from the CUDA
 activity that torch's profiler records."""
+import numpy as np
 import pytest
 
 import emptyroom_b200 as er
@@ -52,3 +53,17 @@ def test_autotuner_times_what_the_plan_runs(n, split):
             plans[0].close()
             fw.release()
         assert _variants(names) == {(4, division), (8, 1)}
+
+
+@pytest.mark.parametrize("edge, n, sigma, dims, kernel", [
+    (25.8, 424, 3.5, 65, "acc_mark_kernel"), (12.0, 259, 3.7, 65, "acc_mark_kernel"),
+    (8.0, 76, 3.7, 65, "acc_points_kernel"), (6.0, 32, 7.0, 33, "acc_points_kernel")])
+def test_accessibility_of_many_overlaps_goes_by_points(ctx, edge, n, sigma, dims, kernel):
+    """Where every point lies in dozens of boxes, testing it against the images until
+    one covers it is faster than marking every box."""
+    t = np.diag([edge] * 3)
+    frac = np.random.default_rng(1).random((n, 3))
+    fw = ctx.upload(er.particles(frac, 50.0, sigma ** 2), t, er.replication_factors(t, 12.5), 12.5 ** 2)
+    names = _kernels(ctx, lambda: ctx.accessibility(fw, (dims,) * 3))
+    fw.release()
+    assert [k for k in ("acc_mark_kernel", "acc_points_kernel") if any(k in x for x in names)] == [kernel]

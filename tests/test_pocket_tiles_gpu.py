@@ -45,3 +45,11 @@ def test_more_links_than_the_first_copy(ctx):
     """A checkerboard: isolated points, more than 2048 distinct face links."""
     i, j, k = np.indices((3, 71, 71))
     _check(ctx, np.where((i + j + k) % 2 == 0, -T, 16 * T))
+
+
+@pytest.mark.parametrize("open_share", [0.25, 0.31, 0.34])
+def test_many_links_between_few_roots(ctx, open_share):
+    """About where the open points percolate: thousands of links, of roots that have
+    one and of roots that have hundreds, channels and pockets among them."""
+    rng = np.random.default_rng(7)
+    _check(ctx, np.where(rng.random((66, 64, 65)) < open_share, -T, 16 * T))

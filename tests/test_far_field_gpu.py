@@ -6,7 +6,9 @@ import numpy as np
 import pytest
 
 import emptyroom_b200 as er
-from emptyroom_b200 import synth
+import oracle
+from conftest import grid_errors, rotated_cell
+from emptyroom_b200 import serve, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +81,72 @@ def test_far_field_of_large_sigma(ctx, sigma, spacing):
     fw.release()
     assert int(ok.sum()) > 500
     assert rms[1] <= 2.0 * rms[0]
+
+
+@pytest.mark.parametrize("abc, angles, n, dims, rotation", [
+    ((14.0, 11.0, 12.0), SKEWED, 25, (111, 100, 118), None),
+    ((14.0, 11.0, 12.0), SKEWED, 25, (111, 100, 118), 3),
+    ((16.0, 14.0, 15.0), CUBIC, 60, (129, 113, 121), 5),
+])
+def test_far_field_at_moderate_energies(ctx, abc, angles, n, dims, rotation):
+    """The energies between the deep and the steep ones too, and cell matrices that
+    are not upper triangular: the grid tolerances of the parity tests, on points of
+    every kind (the FP64 grid as reference)."""
+    import torch
+    f = synth.make_framework(700 + n, abc, angles, n, probe="Xe")
+    P = f.particles()
+    t = f.t_matrix if rotation is None else rotated_cell(f.t_matrix, rotation)
+    fw = ctx.upload(P, t, f.rep, f.rc2)
+    out = torch.empty(dims, dtype=torch.float32, device="cuda")
+    plan = ctx.batch_plan([(fw, dims, out.data_ptr())], er.ER_BATCH_PERSISTENT)
+    assert plan.tile(0) == 8  # chosen only where there is a far field
+    plan.close()
+    e = ctx.grid(fw, dims)
+    ref = ctx.grid(fw, dims, precision=er.ER_PREC_FP64, f64=True)
+    fw.release()
+    rng = np.random.default_rng(8)
+    moderate = np.flatnonzero(((ref >= -10.0) & (ref <= 1e3)).ravel())
+    assert len(moderate) > 2000
+    pick = np.concatenate([rng.choice(moderate, 2000, replace=False), rng.integers(0, ref.size, 3000)])
+    pts = np.stack(np.unravel_index(pick, dims), axis=1) / (np.array(dims) - 1.0)
+    S = oracle.points_abs(P, t, f.rep, f.rc2, pts)
+    st = grid_errors(e.ravel()[pick], ref.ravel()[pick], S)
+    assert st["neg_ok"] and st["pos_ok"] and st["cap_ok"], st
+
+
+def test_far_field_through_every_entry_point(ctx):
+    """A fine grid has the same bits from a single call, a batch copied to the host,
+    the server and the blocking grid of a Widom batch."""
+    import torch
+    dims, T = (129, 65, 97), 298.0
+    fs = [synth.make_framework(720 + k, (9.0, 8.5, 9.5), (85.0, 97.0, 90.0), 16 + 3 * k, probe="Kr")
+          for k in range(3)]
+    fws = [ctx.upload(f.particles(), f.t_matrix, f.rep, f.rc2) for f in fs]
+    single = [ctx.grid(w, dims) for w in fws]
+    out = torch.empty(dims, dtype=torch.float32, device="cuda")
+    plan = ctx.batch_plan([(fws[0], dims, out.data_ptr())], er.ER_BATCH_PERSISTENT)
+    assert plan.tile(0) == 8
+    plan.close()
+
+    hosts = [torch.empty(dims, dtype=torch.float32, pin_memory=True) for _ in fws]
+    ctx.grid_batch([(w, dims, h.data_ptr()) for w, h in zip(fws, hosts)],
+                   er.ER_BATCH_PERSISTENT | er.ER_BATCH_HOST_OUT)
+    for h, s in zip(hosts, single):
+        assert np.array_equal(h.numpy(), s)
+        h.zero_()
+
+    descs = [serve.framework_desc(f.particles(), f.t_matrix, f.rep, f.rc2) for f in fs]
+    with serve.Server(ctx, 4 << 30, slots=3) as srv:
+        tickets = [srv.submit_grid(k, d, dims, h.data_ptr()) for k, (d, h) in enumerate(zip(descs, hosts))]
+        assert all(srv.wait(t)["status"] == 0 for t in tickets)
+    for h, s in zip(hosts, single):
+        assert np.array_equal(h.numpy(), s)
+
+    got, pockets = ctx.henry_batch(fws, T, 20000, [1, 2, 3], block_dims=dims)
+    for k, (w, s) in enumerate(zip(fws, single)):
+        grid = torch.from_numpy(s).cuda()
+        mask = torch.empty(dims, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        assert ctx.block_pockets_device(grid.data_ptr(), dims, T, mask.data_ptr()) == pockets[k]
+        assert ctx.henry_device_mask(w, T, 20000, k + 1, mask.data_ptr(), dims) == got[k]
+        w.release()

@@ -88,13 +88,6 @@ int set_error(er_ctx* ctx, int status, const std::string& msg) {
     return status;
 }
 
-int take_fault(er_ctx* ctx) {
-    if (!ctx->fault_host || !*(volatile int*)ctx->fault_host) return ER_OK;
-    *(volatile int*)ctx->fault_host = 0;
-    return set_error(ctx, ER_ERR_CUDA,
-                     "a kernel's bounded wait gave up; what its blocks compute was not written");
-}
-
 int cuda_error(er_ctx* ctx, cudaError_t e, const char* what) {
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
     cudaGetLastError();
@@ -553,7 +546,7 @@ const char* er_ctx_last_error(const er_ctx* ctx) { return ctx ? ctx->last_error.
 
 int er_ctx_synchronize(er_ctx* ctx) {
     if (!ctx) return ER_ERR_INVALID;
-    ER_SYNC(ctx, ctx->stream);
+    ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return ER_OK;
 }
 
@@ -781,7 +774,7 @@ int er_grid(er_ctx* ctx, int fw_id, int nx, int ny, int nz, int flags, void* out
         if (!dev_out) {
             ER_CUDA(ctx, cudaMemcpyAsync(out, d64, npts * sizeof(double), cudaMemcpyDeviceToHost,
                                          ctx->stream));
-            ER_SYNC(ctx, ctx->stream);
+            ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         }
         return ER_OK;
     }
@@ -805,13 +798,13 @@ int er_grid(er_ctx* ctx, int fw_id, int nx, int ny, int nz, int flags, void* out
         if (!f64) {
             ER_CUDA(ctx, cudaMemcpyAsync(out, dst, npts * sizeof(float), cudaMemcpyDeviceToHost,
                                          ctx->stream));
-            ER_SYNC(ctx, ctx->stream);
+            ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         } else {
             // D2H as float (half the bytes), widen on the host
             float* tmp = (float*)out;  // the first half of the caller's double buffer
             ER_CUDA(ctx, cudaMemcpyAsync(tmp, dst, npts * sizeof(float), cudaMemcpyDeviceToHost,
                                          ctx->stream));
-            ER_SYNC(ctx, ctx->stream);
+            ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
             double* o = (double*)out;
             for (size_t i = npts; i-- > 0;) o[i] = (double)tmp[i];
         }
@@ -840,7 +833,7 @@ int er_grid_sheet(er_ctx* ctx, int fw_id, int nx, int ny, int nz, int x_index,
         return set_error(ctx, ER_ERR_NOMEM, "sheet: pinned staging failed");
     ER_CUDA(ctx, cudaMemcpyAsync(ctx->pinned.ptr, (float*)c.grid.ptr + (size_t)x_index * ns,
                                  ns * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    ER_SYNC(ctx, ctx->stream);
+    ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const float* src = (const float*)ctx->pinned.ptr;
     for (size_t i = 0; i < ns; ++i) out_sheet[i] = (double)src[i];
     return ER_OK;
@@ -1145,7 +1138,7 @@ int er_grid_batch(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode) {
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->copy_stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) return cuda_error(ctx, e, "batch: run / copy-out");
-        return take_fault(ctx);
+        return ER_OK;
     }
     // run once: the launches go straight to the stream (capturing and
     // instantiating a graph for one replay took 130 us of a call)
@@ -1155,7 +1148,6 @@ int er_grid_batch(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode) {
     st = plan_enqueue(p);
     if (st == ER_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess)
         st = cuda_error(ctx, cudaGetLastError(), "batch: run");
-    if (st == ER_OK) st = take_fault(ctx);
     er_batch_plan_destroy(p);
     return st;
 }
@@ -1217,39 +1209,47 @@ extern "C" int er_probe_rcp64_seed(er_ctx* ctx, double* max_rel_err) {
     ER_CUDA(ctx, cudaGetLastError());
     unsigned long long h = 0;
     ER_CUDA(ctx, cudaMemcpyAsync(&h, bits, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    ER_SYNC(ctx, ctx->stream);
+    ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     double v;
     memcpy(&v, &h, sizeof(v));
     *max_rel_err = v;
     return ER_OK;
 }
 
-// One CTA waits, with the engine's bounded wait, for an mbarrier phase that
-// nothing completes (no arrival, no copy); when the wait gives up it raises
-// the fault word.
+// One CTA waits for an mbarrier phase that nothing completes (no arrival, no
+// copy), `spins` polls at most, and raises the fault word when it has given up.
+// (The library's other kernels wait for nothing but their own block.)
 __global__ void wait_timeout_kernel(int spins, int* fault) {
     __shared__ unsigned long long bar;
+    const unsigned a = (unsigned)__cvta_generic_to_shared(&bar);
     if (threadIdx.x == 0) {
-        mbar_init(&bar);
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const bool gave_up = !mbar_wait(&bar, 0u, spins);
-    if (__syncthreads_or(gave_up) && threadIdx.x == 0) {
+    unsigned done = 0;
+    for (int i = 0; i < spins && !done; ++i)
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(a)
+            : "memory");
+    if (__syncthreads_or(!done) && threadIdx.x == 0) {
         atomicExch(fault, 1);
-        mbar_inval(&bar);
+        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(a) : "memory");
     }
 }
 
 extern "C" int er_selftest_wait_timeout(er_ctx* ctx, int spins) {
     if (!ctx || spins < 1) return ER_ERR_INVALID;
     ER_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (int st = take_fault(ctx)) return st;  // an earlier fault is reported first
+    volatile int* fault = ctx->fault_host;
+    *fault = 0;
     wait_timeout_kernel<<<1, 64, 0, ctx->stream>>>(spins, ctx->fault_dev);
     ER_CUDA(ctx, cudaGetLastError());
     ER_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (take_fault(ctx) == ER_OK)
-        return set_error(ctx, ER_ERR_CUDA, "selftest: the bounded wait did not report");
+    if (!*fault) return set_error(ctx, ER_ERR_CUDA, "selftest: the bounded wait did not report");
     return ER_OK;
 }
 

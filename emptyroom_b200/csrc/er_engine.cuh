@@ -202,33 +202,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return y;
 }
 
-// ------------------------------------------------ bounded mbarrier wait
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_inval(unsigned long long* bar) {
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Waits for the phase of `parity` to complete; false after `spins` polls (the
-// caller records the fault instead of hanging).
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, int spins) {
-    const unsigned a = smem_u32(bar);
-    for (int i = 0; i < spins; ++i) {
-        unsigned done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
 // Sum of the warps' counts below this warp's; *total gets the sum of all. One
 // barrier per call: consecutive calls use `buf` 0 and 1 in turn, so a warp
 // writes a buffer again only after the barrier of the call between, which
@@ -635,13 +608,6 @@ __device__ __forceinline__ void fold_packed(EngineSmem& s, f2_t* acc2) {
         tot_at(s, 2 * m + 1) += (double)a1;
         acc2[m] = 0ull;
     }
-}
-
-__device__ __forceinline__ void cta_centre(const EngineSmem& s, double& o0, double& o1,
-                                           double& o2) {
-    o0 = s.org[0];
-    o1 = s.org[1];
-    o2 = s.org[2];
 }
 
 // Lattice inner list: every pair inside the cutoff, packed over point pairs.

@@ -467,11 +467,11 @@ int er_probe_fp32_rate(er_ctx* ctx, double seconds, double* instr_per_s);
  * error is the square of this. No counterpart in the reference (FP64 `/`). */
 int er_probe_rcp64_seed(er_ctx* ctx, double* max_rel_err);
 
-/* Self-test of the kernels' bounded waits: one CTA waits, `spins` polls at
- * most, for a completion barrier that nothing completes; the wait must give
- * up, raise the context's fault word and let the host see it (ER_OK then;
- * ER_ERR_CUDA if it did not report). The context stays usable. No counterpart
- * in the reference. */
+/* Self-test of a bounded wait on the device (none of the library's own kernels
+ * waits for another block or a copy): one CTA waits, `spins` polls at most, for
+ * a completion barrier that nothing completes; the wait must give up, raise the
+ * context's fault word and let the host see it (ER_OK then; ER_ERR_CUDA if it
+ * did not report). The context stays usable. No counterpart in the reference. */
 int er_selftest_wait_timeout(er_ctx* ctx, int spins);
 
 /* Library version string. */

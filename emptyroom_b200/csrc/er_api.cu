@@ -308,8 +308,10 @@ static int64_t task_bricks(const GridTask& t) { return (int64_t)t.nb[0] * t.nb[1
 // CTAs per brick of a P = 4 grid: 4 while they have an SM each, 2 while they
 // fit the three slots an SM has, 1 from there on (a second wave of split CTAs
 // costs more than the idle slots). Same bits in every case. Measured unsplit /
-// 2 / 4, us a call, 424-atom cell: 16^3 136 / 77 / 66, 32^3 (32 bricks) 55 / 41
-// / 37, 40^3 (75) 51 / 43 / 53, 56^3 (196) 59 / 54 / 76, 64^3 (256) 56 / 68 / 95.
+// 2 / 4, us a call and its wait, 424-atom cell: 16^3 144 / 89 / 68, 32^3 (32
+// bricks) 66 / 53 / 43, 40^3 (75) 61 / 57 / 62, 56^3 (196) 71 / 66 / 84, 64^3 (256)
+// 68 / 82 / 99; 2000-atom cell: 32^3 230 / 146 / 107, 40^3 192 / 154 / 163, 56^3 206
+// / 178 / 225, 64^3 193 / 226 / 280.
 static int grid_split(const er_ctx* ctx, int64_t bricks) {
     if (4 * bricks <= ctx->num_sms) return 4;
     return 2 * bricks <= 3 * ctx->num_sms ? 2 : 1;

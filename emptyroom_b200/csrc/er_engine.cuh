@@ -1685,8 +1685,9 @@ __device__ void process_cta(const Pol& pol, const FwDev& fw, const CutoffConsts&
         __syncthreads();
     }
     const float R2f = (float)(cc.rcm * cc.rcm);
-    // rows are pruned in FP32 with a millimetre of slack in a metre: every
-    // image that passes the test below lies in the pruned range
+    // rows are pruned in FP32 with 1e-3 A of slack, some hundred times the rounding
+    // of these coordinates (|x| < 64 A: 4e-6 A): every image that passes the test
+    // below lies in the pruned range
     const float Rrow = (float)cc.rcm + 1e-3f, R2row = Rrow * Rrow;
     // Fills the candidate list, flushes it and goes on until every row is done.
     // One flush site (the pair loops are inlined there), and a chunk of images

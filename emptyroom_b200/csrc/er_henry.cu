@@ -683,11 +683,13 @@ int henry_enqueue(er_ctx* ctx, const FwRecord& fw, double temperature, int n, ui
         if (e == cudaSuccess) kernel<<<ecta * split, kThreads, sizeof(EngineSmem), st>>>(task);
         return e;
     };
-    // runs of few CTAs share each CTA's points among several (same bits): four
-    // while a CTA has an SM, two while the halves fit an SM's two slots.
-    // Measured whole / 2 / 4, us a call, 424-atom cell: 16k insertions 187 /
-    // 143 / 127, 32k 169 / 136 / 126, 65k 149 / 125 / 126, 100k 139 / 135 / 149,
-    // 150k 138 / 137 / 162, 400k 192 / 212 / 265.
+    // runs of few CTAs share each CTA's points among several (same bits, compared
+    // for thirteen sizes from 1 to 4e5 in both cells below): four while a CTA has an
+    // SM, two while the halves fit an SM's two slots. Measured whole / 2 / 4, us a
+    // call, 424-atom cell: 16k insertions 157 / 114 / 96, 33k 133 / 111 / 96, 76k 115
+    // / 99 / 101, 100k 110 / 110 / 122, 150k 113 / 115 / 136, 400k 178 / 202 / 250;
+    // 2000-atom cell: 16k 515 / 337 / 232, 76k 331 / 245 / 233, 100k 282 / 258 / 263,
+    // 150k 283 / 250 / 305, 400k 444 / 463 / 573.
     if (hp == kHenryP) ER_CUDA(ctx, energy(henry_energy_kernel<kHenryP, 1>, 1));
     else if (2 * ecta <= ctx->num_sms)
         ER_CUDA(ctx, energy(henry_energy_kernel<kHenryPSmall, 4>, 4));
@@ -823,8 +825,9 @@ namespace {
 constexpr int kHenryPipes = 6;
 
 // Device bytes one pipeline holds for a job: 40 per insertion (Cartesian
-// FP64 point, bin key, order, scan scratch, FP32 energy), 24 per blocking-grid
-// point (FP32 grid, mask, pocket labels and segments), plus the bin tables.
+// FP64 point, bin key, order, scatter scratch, FP32 energy), at most 24 per
+// blocking-grid point (FP32 grid, mask and pocket labels 9, the link set 24 to 40
+// per point of three faces), plus the bin tables.
 size_t henry_pipe_bytes(int64_t n_ins, const int bd[3]) {
     return 40 * (size_t)n_ins + 24 * (size_t)bd[0] * bd[1] * bd[2] + ((size_t)64 << 20);
 }

@@ -45,3 +45,14 @@ def test_widom_mask_rows(ctx, dims):
     o = oracle.henry(P, f.t_matrix, f.rep, f.rc2, T, 78, 4096, mask=mask, want_energies=True)
     assert r["n_blocked"] == o["n_blocked"] > 0
     assert np.array_equal(np.isinf(r["energies"]), np.isinf(o["energies"]))
+
+
+@pytest.mark.parametrize("n", [999_999, 10**6])
+def test_widom_at_the_line_between_warp_sizes(ctx, n):
+    f = synth.make_framework(13, (17.0, 15.0, 19.0), (75.0, 102.0, 96.0), 80, probe="Xe")
+    P = f.particles()
+    fw = ctx.upload(P, f.t_matrix, f.rep, f.rc2)
+    r = ctx.henry(fw, T, n, seed=79)
+    fw.release()
+    o = oracle.henry_cells(P, f.t_matrix, f.rep, f.rc2, T, 79, n)
+    assert abs(r["sum_w"] - o["sum_w"]) <= 1e-6 * o["sum_w"]

@@ -415,6 +415,9 @@ def run_ours(args, ws, rank, local, pg):
     roof = {"bound": "fp32", "achieved": achieved / 1e12, "peak": fp32_rate / 1e12,
             "unit": "Tinst/s", "frac": achieved / fp32_rate,
             "peak_source": "measured FP32 FFMA issue rate (er_probe_fp32_rate) on this GPU",
+            "basis": f"{PAIR_INSTR} instructions credited per in-cutoff pair, the interpolated pairs of "
+                     "a far field too: a credited rate, not the pipe's utilisation "
+                     "(comp.roofline_frac: every pair evaluated)",
             "traffic": load_traffic(points_step)}
     # the grid store against the measured HBM copy bandwidth (not the bound)
     roof["grid_store_gbs"] = 4.0 * points_step / t_kernel / 1e9
@@ -826,9 +829,9 @@ def run_serving(ctx, args):
 
 def load_traffic(points_step):
     """DRAM bytes per launch of the batch kernel from the committed ncu
-    capture of a smaller batch (profiles/grid_persistent_traffic.json), scaled
+    capture of a smaller batch (profiles/grid_batch_traffic.json), scaled
     to this launch by grid points (the traffic is the grid store)."""
-    p = os.path.join(ROOT, "profiles", "grid_persistent_traffic.json")
+    p = os.path.join(ROOT, "profiles", "grid_batch_traffic.json")
     if not os.path.exists(p):
         return None
     d = json.load(open(p))

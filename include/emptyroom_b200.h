@@ -93,9 +93,14 @@ int er_framework_bytes(er_ctx* ctx, int fw_id, size_t* bytes);
 #define ER_PREC_NEAR64 0x0  /* default: FP32 pair terms except the pairs of atoms within
                                 5 A of a warp's points, which are FP64 (the large terms
                                 whose FP32 rounding dominates where terms cancel); FP32
-                                sums of 16 terms (64 on the cutoff shell) folded into
-                                FP64 per-point totals. Within 1e-5 relative of FP64 on
-                                points with E < -10 K */
+                                sums of 8 or 16 terms (64 on the cutoff shell) folded
+                                into FP64 per-point totals; on fine grids the sum over
+                                the atoms far from a brick is interpolated in FP64 from
+                                fewer points, which adds less than the FP32 terms'
+                                rounding. Within 1e-5 relative of FP64 on points with
+                                E < -10 K for mixed sigmas up to 3.5 A or so; larger ones
+                                leave steep terms beyond the 5 A (pores in walls of
+                                atoms all at 4 A: up to 2.5e-5, all at 6 A: 4e-4) */
 #define ER_PREC_COMP 0x08    /* all pair terms FP32, FP32 sums of 64 terms folded into
                                 FP64 per-point totals: faster, but its error on E < 0
                                 points reaches ~2e-5 relative where large near terms

@@ -258,31 +258,52 @@ static float far_distance2(const FwRecord& fw, const GridTask& t, double* diag =
     return rf + sqrt(diag2) < sqrt(fw.rc2) ? (float)(rf * rf) : 0.f;
 }
 
-// P = 8 where its bricks have a far field of 32 atoms or more (the nodes and
-// barriers of a smaller one cost what it saves) and are enough to fill the GPU:
-// half its CTA slots while the spacing is fine, all of them where the far field
-// is small. Measured P = 4 / 8, us a call: 8 A cell at 0.1 A (250 bricks) 235 / 174,
-// 10 A at 0.13 A (250) 243 / 233, 14 A at 0.18 A (250) 265 / 286; 25.8 A cell of
-// 424 atoms at 0.17 A (1900) 385 / 375, at 0.15 A 553 / 474; of 2500 atoms at 0.17
-// A 2019 / 1897, at 0.13 A 4231 / 3093; of 150 atoms at 0.17 A (18 far atoms) 186
-// / 198, at 0.15 A (29) 266 / 266, at 0.12 A (41) 523 / 497.
-int default_tile(const er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, int prec) {
-    if (prec != PREC_NEAR64) return 4;
+// Time of a P = 8 grid point over that of P = 4 where both fill the GPU, by the
+// volume of the far shell and its atoms (fitted to 1,120 random grids, see
+// default_tile): 1 and more where there is no far field, or one of fewer than 32
+// atoms (the nodes and barriers of a smaller one cost what it saves).
+static double far_share(const FwRecord& fw, int nx, int ny, int nz) {
     GridTask t;
     t.tile_p = 8;
     t.nx = nx; t.ny = ny; t.nz = nz;
     double diag = 0.0;
     const double rf = sqrt((double)far_distance2(fw, t, &diag));
-    if (!(rf > 0.0)) return 4;
+    if (!(rf > 0.0)) return 2.0;
     // a shell about the brick, from Rf outside it to rc from its far corners
-    const double in = rf + diag / 4.0, out = sqrt(fw.rc2) - diag / 2.0;
-    const double far_atoms =
-        4.18879 * (out * out * out - in * in * in) * fw.n_atoms / std::max(fw.volume, 1e-9);
-    if (!(far_atoms >= 32.0)) return 4;
-    const int64_t bricks = (int64_t)((nx + 15) / 16) * ((ny + 7) / 8) * ((nz + 15) / 16);
-    const double h = std::max(fw.cell_len[0] / (nx - 1), fw.cell_len[2] / (nz - 1));
-    const int64_t slots = 3 * ctx->num_sms;
-    return bricks >= (h <= 0.14 ? slots / 2 : slots) ? 8 : 4;
+    const double rc = sqrt(fw.rc2), in = rf + diag / 4.0, out = rc - diag / 2.0;
+    const double shell = out * out * out - in * in * in;
+    const double atoms = 4.18879 * shell * fw.n_atoms / std::max(fw.volume, 1e-9);
+    if (!(atoms >= 32.0)) return 2.0;
+    return 0.964 - 0.43 * shell / (rc * rc * rc) + 3.9 / atoms;
+}
+
+// Time of a launch of equal bricks, in launches that give every SM its three CTAs:
+// one or two CTAs on an SM run faster than three (measured on 8 x 16-line grids
+// of 74 to 1340 bricks: 0.60 with one on the busiest SM, 0.78 with two, 1.00, then
+// 1.39, 1.60, 1.85, 2.17, ...).
+static double launch_time(const er_ctx* ctx, int64_t bricks) {
+    const int64_t c = (bricks + ctx->num_sms - 1) / ctx->num_sms;  // on the busiest SM
+    const double full = (double)(c / 3);
+    return c % 3 == 0 ? 0.15 + 0.85 * full : c % 3 == 1 ? 0.60 + 0.785 * full : 0.78 + 0.82 * full;
+}
+
+// P = 8 where a far field saves more than the larger bricks lose at the end of the
+// launch. Over 1,120 random grids (cells of 6-40 A, 20-5000 atoms, 0.06-0.21 A, 30 to
+// 4500 P = 8 bricks) the time over that of P = 4 is 0.874 in the geometric mean
+// (always the faster one: 0.870), 24 grids are more than 2 % slower, by 17 % at most.
+// A line at half the CTA slots (spacings up to 0.14 A) or all of them gave 0.882 and
+// 135, by up to 28 %: 450 bricks on 444 slots take nearly as long as 888 (94 x 200 x
+// 47 points at 0.17 A 709 us with P = 4, 832 with P = 8).
+constexpr double kTile8Gain = 0.96;
+
+int default_tile(const er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, int prec) {
+    if (prec != PREC_NEAR64) return 4;
+    const double share = far_share(fw, nx, ny, nz);
+    if (!(share < 1.0)) return 4;
+    const int64_t across = ((int64_t)ny + 7) / 8 * (((int64_t)nz + 15) / 16);
+    const int64_t b4 = ((int64_t)nx + 7) / 8 * across, b8 = ((int64_t)nx + 15) / 16 * across;
+    if (2 * b4 <= 3 * ctx->num_sms) return 4;  // P = 4 divides its bricks (grid_split)
+    return 2.0 * share * launch_time(ctx, b8) < kTile8Gain * launch_time(ctx, b4) ? 8 : 4;
 }
 
 int fill_grid_task(er_ctx* ctx, const FwRecord& fw, int nx, int ny, int nz, float* out,
@@ -912,6 +933,12 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
     p->prec = prec;
     p->n_jobs = n_jobs;
     std::vector<double> cost;
+    // whether the jobs, in one launch, fill the GPU several times over at P = 8
+    int64_t bricks8 = 0;
+    for (int i = 0; i < n_jobs; ++i)
+        bricks8 += ((int64_t)jobs[i].nx + 15) / 16 * (((int64_t)jobs[i].ny + 7) / 8) *
+                   (((int64_t)jobs[i].nz + 15) / 16);
+    const bool filled = mode == ER_BATCH_PERSISTENT && bricks8 >= 12 * ctx->num_sms;
     for (int i = 0; i < n_jobs; ++i) {
         const FwRecord* f = find_fw(ctx, jobs[i].fw_id);
         if (!f || !jobs[i].out_device) {
@@ -924,10 +951,15 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
         const bool dims_ok = jobs[i].nx >= 2 && jobs[i].ny >= 2 && jobs[i].nz >= 2;
         if (dims_ok)
             tile_p = default_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, prec);
-        // (a far field needs P = 8 and always pays: nothing to time)
-        if (autotune && dims_ok && tile_p == 4)
-            st = tune_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device, prec,
-                           mode == ER_BATCH_PERSISTENT, &tile_p);
+        // (a far field needs P = 8; where it pays there is nothing to time)
+        if (autotune && dims_ok && tile_p == 4) {
+            if (filled && prec == PREC_NEAR64 &&
+                far_share(*f, jobs[i].nx, jobs[i].ny, jobs[i].nz) < kTile8Gain)
+                tile_p = 8;
+            else
+                st = tune_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device,
+                               prec, mode == ER_BATCH_PERSISTENT, &tile_p);
+        }
         GridTask t;
         if (st == ER_OK)
             st = fill_grid_task(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device, t,

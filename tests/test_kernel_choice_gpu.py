@@ -67,3 +67,21 @@ def test_accessibility_of_many_overlaps_goes_by_points(ctx, edge, n, sigma, dims
     names = _kernels(ctx, lambda: ctx.accessibility(fw, (dims,) * 3))
     fw.release()
     assert [k for k in ("acc_mark_kernel", "acc_points_kernel") if any(k in x for x in names)] == [kernel]
+
+
+@pytest.mark.parametrize("dims, tile", [((94, 200, 47), 4),    # 450 bricks of P = 8 on 444 CTA slots
+                                        ((94, 200, 94), 8),    # twice as many
+                                        ((80, 80, 80), 8)])    # 250: two on most SMs, 500 of P = 4
+def test_larger_bricks_where_their_launch_ends_well(ctx, dims, tile):
+    """A far field is worth P = 8 unless its few bricks leave most of the last wave
+    idle (the spacing is 0.13 A in each case)."""
+    import torch
+    abc = tuple(0.13 * (d - 1) for d in dims)
+    f = synth.make_framework(31, abc, (90.0, 90.0, 90.0), int(0.03 * np.prod(abc)))
+    fw = ctx.upload(f.particles(), f.t_matrix, f.rep, f.rc2)
+    out = torch.empty(dims, dtype=torch.float32, device="cuda")
+    plan = ctx.batch_plan([(fw, dims, out.data_ptr())], er.ER_BATCH_PERSISTENT)
+    got = plan.tile(0)
+    plan.close()
+    fw.release()
+    assert got == tile

@@ -388,9 +388,13 @@ int launch_grid_batch(er_ctx* ctx, const GridTask* d_tasks, const int* d_start, 
 // precision mode, form). It times the kernels that the plan will launch: the
 // bricks of a batch in one launch (`one_launch`) are not divided among CTAs,
 // those of a launch of their own are where they are few. The form holds that
-// division and whether P = 8 has a far field.
+// division, whether P = 8 has a far field and, for jobs of less than four waves of
+// P = 8 bricks, the bricks per SM of both variants: what is faster for a job that
+// fills the GPU is not for a small one on its own (118 x 37 x 36 points 240 us with P =
+// 4, 357 with P = 8). Among other jobs that fill it (`filled`) a small job takes the
+// verdict of a large one of its class if there is one.
 int tune_tile(er_ctx* ctx, const FwRecord& f, int nx, int ny, int nz, float* out, int prec,
-              bool one_launch, int* tile_p) {
+              bool one_launch, bool filled, int* tile_p) {
     GridTask task[2];  // P = 4, P = 8
     for (int v = 0; v < 2; ++v)
         if (int st = fill_grid_task(ctx, f, nx, ny, nz, out, task[v], 4 << v)) return st;
@@ -399,10 +403,21 @@ int tune_tile(er_ctx* ctx, const FwRecord& f, int nx, int ny, int nz, float* out
     const int dims[3] = {nx, ny, nz};
     for (int d = 0; d < 3; ++d) h = std::min(h, f.cell_len[d] / std::max(dims[d] - 1, 1));
     const int split = one_launch ? 1 : grid_split(ctx, task_bricks(task[0]));
-    const std::tuple<int, int, int, int, int> key(
-        (int)lround(2.0 * log2(rho)), (int)lround(4.0 * log2(h)), (int)lround(4.0 * sqrt(f.rc2)),
-        prec, 2 * split + (task[1].far2 > 0.f ? 1 : 0));
-    auto it = ctx->tune.find(key);
+    const int slots = 3 * ctx->num_sms;
+    const auto per_sm = [&](const GridTask& t) {  // at most 12 of P = 8, 24 of P = 4
+        return (int)((task_bricks(t) + ctx->num_sms - 1) / ctx->num_sms);
+    };
+    const bool small = task_bricks(task[1]) < 4 * slots;
+    auto key_of = [&](int bricks) {
+        return std::tuple<int, int, int, int, int>(
+            (int)lround(2.0 * log2(rho)), (int)lround(4.0 * log2(h)),
+            (int)lround(4.0 * sqrt(f.rc2)), prec,
+            16 * bricks + 2 * split + (task[1].far2 > 0.f ? 1 : 0));
+    };
+    const auto key = key_of(small ? 32 * per_sm(task[0]) + per_sm(task[1]) : 0);
+    auto it = ctx->tune.end();
+    if (filled) it = ctx->tune.find(key_of(0));
+    if (it == ctx->tune.end()) it = ctx->tune.find(key);
     if (it != ctx->tune.end()) {
         *tile_p = it->second;
         return ER_OK;
@@ -416,7 +431,6 @@ int tune_tile(er_ctx* ctx, const FwRecord& f, int nx, int ny, int nz, float* out
     // enough for four waves of the bigger (P = 8) bricks on this GPU, so that
     // neither is timed on an underfilled launch (a smaller grid is timed whole).
     const int nbyz = ((ny + 2 * kWJ - 1) / (2 * kWJ)) * ((nz + 2 * kWK - 1) / (2 * kWK));
-    const int slots = 3 * ctx->num_sms;
     const int layers = 16 * std::max(1, (4 * slots + nbyz - 1) / nbyz);
     for (int P : {4, 8}) {
         GridTask& t = task[P / 8];
@@ -958,7 +972,7 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
                 tile_p = 8;
             else
                 st = tune_tile(ctx, *f, jobs[i].nx, jobs[i].ny, jobs[i].nz, jobs[i].out_device,
-                               prec, mode == ER_BATCH_PERSISTENT, &tile_p);
+                               prec, mode == ER_BATCH_PERSISTENT, filled, &tile_p);
         }
         GridTask t;
         if (st == ER_OK)

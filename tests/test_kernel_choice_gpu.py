@@ -85,3 +85,21 @@ def test_larger_bricks_where_their_launch_ends_well(ctx, dims, tile):
     plan.close()
     fw.release()
     assert got == tile
+
+
+def test_a_small_job_is_not_tuned_by_a_large_one(ctx):
+    """Two jobs of one density and spacing: the large one may run 8 points per thread,
+    the small one on its own, whose bricks would halve to 20, may not."""
+    import torch
+    f = synth.make_framework(32, (32.0, 32.0, 32.0), (90.0, 90.0, 90.0), 810)
+    with er.Context(0) as own:  # nothing tuned yet
+        fw = own.upload(f.particles(), f.t_matrix, f.rep, f.rc2)
+        out = torch.empty((160,) * 3, dtype=torch.float32, device="cuda")
+        tiles = []
+        for dims in ((160, 160, 160), (160, 16, 16)):
+            plan = own.batch_plan([(fw, dims, out.data_ptr())],
+                                  er.ER_BATCH_PERSISTENT | er.ER_BATCH_AUTOTUNE | er.ER_BATCH_COMP)
+            tiles.append(plan.tile(0))
+            plan.close()
+        fw.release()
+    assert tiles[0] in (4, 8) and tiles[1] == 4

@@ -880,15 +880,18 @@ __global__ void __launch_bounds__(256)
 // Marking takes c tests a point, c = the boxes that lie over it (27 images: at most
 // 3 along an axis); a point takes some multiple of 27 n / c images until one covers
 // it. So c^2 / n decides, at 18 (grids of few points, whose blocks are too few to
-// hide a point's chain of tests, 48). Measured boxes / points, us a call: 424 atoms
+// hide a point's chain of tests, 48; fewer than 16 atoms, whose chains are short and
+// whose boxes are few for the GPU, 8). Measured boxes / points, us a call: 424 atoms
 // in 25.8 A, sigma 3.5 A (c^2 / n = 0.17), 65^3 71 / 1793; 259 in 12 A, 3.7 A (14),
 // 33^3 50 / 112, 65^3 130 / 197, 129^3 697 / 777; 150 in 10 A, 3.7 A (25) 51 / 76, 128
 // / 118, 709 / 480; 76 in 8 A, 3.7 A (48) 55 / 56, 133 / 85, 689 / 333; 76 in 8 A, 7 A
-// (2183) 131 / 34, 529 / 61, 3547 / 214.
+// (2183) 131 / 34, 529 / 61, 3547 / 214; 4 in 6 A, 3 A (4) 43 / 43, 65 / 72, 261 / 275,
+// 3.7 A (14) 48 / 37, 84 / 60, 331 / 224.
 static bool acc_from_points(const FwRecord& f, const double* reach, int64_t points) {
     double c = f.n_atoms;
     for (int d = 0; d < 3; ++d) c *= std::min(2.0 * f.sig_mean * reach[d], 3.0);
-    return c * c > (points < 100000 ? 48.0 : 18.0) * f.n_atoms && f.n_atoms <= INT32_MAX / 27;
+    const double line = f.n_atoms < 16 ? 8.0 : points < 100000 ? 48.0 : 18.0;
+    return c * c > line * f.n_atoms && f.n_atoms <= INT32_MAX / 27;
 }
 
 }  // namespace er

@@ -57,7 +57,8 @@ def test_autotuner_times_what_the_plan_runs(n, split):
 
 @pytest.mark.parametrize("edge, n, sigma, dims, kernel", [
     (25.8, 424, 3.5, 65, "acc_mark_kernel"), (12.0, 259, 3.7, 65, "acc_mark_kernel"),
-    (8.0, 76, 3.7, 65, "acc_points_kernel"), (6.0, 32, 7.0, 33, "acc_points_kernel")])
+    (8.0, 76, 3.7, 65, "acc_points_kernel"), (6.0, 32, 7.0, 33, "acc_points_kernel"),
+    (6.0, 4, 3.7, 65, "acc_points_kernel")])
 def test_accessibility_of_many_overlaps_goes_by_points(ctx, edge, n, sigma, dims, kernel):
     """Where every point lies in dozens of boxes, testing it against the images until
     one covers it is faster than marking every box."""

@@ -153,15 +153,26 @@ __global__ void __launch_bounds__(kThreads, grid_min_blocks<PREC>())
 // as SM slots fall free, which is the work queue: resident CTAs that pulled
 // items from a counter kept their loop's state in registers through the pair
 // loops and ran slower (8 triclinic frameworks, 54 M points: 17.36 against
-// 16.73 ms; 64 grids of 32^3 680 against 633 us a call).
+// 16.73 ms; 64 grids of 32^3 680 against 633 us a call). A launch that the GPU holds
+// at once has no such order: which SM gets a second or third CTA shows only when
+// that CTA starts, and it should find a brick of the grid's end then. There `head`
+// is given and a CTA takes the next brick when it starts (86 x 67 x 35 points, 297
+// bricks on 148 SMs, 337 -> 263 us; 67 x 130 x 24, 306, 383 -> 325; the counter wraps
+// to 0 with the last one, ready for the next replay).
 // With task_left given, the CTA that finishes a task's last brick raises the
 // task's flag in host-mapped memory (done_host), so the host can copy that
 // grid out while the kernel runs on.
 template <int PREC>
 __global__ void __launch_bounds__(kThreads, grid_min_blocks<PREC>())
     grid_batch_kernel(const GridTask* __restrict__ tasks, const int* __restrict__ start,
-                      int n_tasks, int* task_left, volatile int* done_host) {
-    const int item = blockIdx.x;
+                      int n_tasks, unsigned* head, int* task_left, volatile int* done_host) {
+    int item = blockIdx.x;
+    if (head) {
+        int& next = engine_smem().wcnt[0][0];  // written again behind several barriers
+        if (threadIdx.x == 0) next = (int)atomicInc(head, gridDim.x - 1);
+        __syncthreads();
+        item = next;
+    }
     int k = 0;
     for (int hi = n_tasks - 1; k < hi;) {
         const int mid = (k + hi + 1) >> 1;
@@ -364,17 +375,20 @@ int launch_grid_plain(er_ctx* ctx, const GridTask& t, int prec) {
     return launch_grid_plain_on(ctx, t, prec, ctx->stream);
 }
 
+// d_head: a counter at 0, which every launch leaves at 0.
 int launch_grid_batch(er_ctx* ctx, const GridTask* d_tasks, const int* d_start, int n_tasks,
-                      int n_items, int prec, int* task_left = nullptr, int* done_dev = nullptr) {
+                      int n_items, unsigned* d_head, int prec, int* task_left = nullptr,
+                      int* done_dev = nullptr) {
     if (n_items == 0) return ER_OK;
     const size_t smem = sizeof(EngineSmem);
     cudaStream_t st = ctx->stream;
+    unsigned* head = n_items <= 3 * ctx->num_sms ? d_head : nullptr;
     if (prec == PREC_NEAR64)
-        grid_batch_kernel<PREC_NEAR64><<<n_items, kThreads, smem, st>>>(d_tasks, d_start, n_tasks,
-                                                                        task_left, done_dev);
+        grid_batch_kernel<PREC_NEAR64><<<n_items, kThreads, smem, st>>>(
+            d_tasks, d_start, n_tasks, head, task_left, done_dev);
     else
-        grid_batch_kernel<PREC_COMP><<<n_items, kThreads, smem, st>>>(d_tasks, d_start, n_tasks,
-                                                                      task_left, done_dev);
+        grid_batch_kernel<PREC_COMP><<<n_items, kThreads, smem, st>>>(
+            d_tasks, d_start, n_tasks, head, task_left, done_dev);
     ER_CUDA(ctx, cudaGetLastError());
     return ER_OK;
 }
@@ -886,9 +900,10 @@ struct er_batch_plan {
     int n_jobs = 0;
     std::vector<GridTask> tasks;   // job order
     std::vector<int> order;        // queue position -> job (longest first)
-    void* d_block = nullptr;       // one pool allocation: tasks, start
+    void* d_block = nullptr;       // one pool allocation: tasks, start, head
     GridTask* d_tasks = nullptr;   // queue order
     int* d_start = nullptr;        // n_jobs + 1 brick offsets, queue order
+    unsigned* d_head = nullptr;    // the next brick of a small launch
     int n_items = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -919,7 +934,8 @@ static int plan_enqueue(er_batch_plan* p) {
         }
         return ER_OK;
     }
-    return launch_grid_batch(ctx, p->d_tasks, p->d_start, p->n_jobs, p->n_items, p->prec);
+    return launch_grid_batch(ctx, p->d_tasks, p->d_start, p->n_jobs, p->n_items, p->d_head,
+                             p->prec);
 }
 
 }  // namespace er
@@ -949,7 +965,7 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
     std::vector<double> cost;
     // whether the jobs, in one launch, fill the GPU several times over at P = 8
     int64_t bricks8 = 0;
-    for (int i = 0; i < n_jobs; ++i)
+    for (int i = 0; autotune && i < n_jobs; ++i)
         bricks8 += ((int64_t)jobs[i].nx + 15) / 16 * (((int64_t)jobs[i].ny + 7) / 8) *
                    (((int64_t)jobs[i].nz + 15) / 16);
     const bool filled = mode == ER_BATCH_PERSISTENT && bricks8 >= 12 * ctx->num_sms;
@@ -995,7 +1011,7 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
     // queue-ordered tasks and brick offsets, staged in pinned memory, one copy
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t s_tasks = al(std::max(n_jobs, 1) * sizeof(GridTask));
-    const size_t s_start = al((size_t)(n_jobs + 1) * sizeof(int));
+    const size_t s_start = al((size_t)(n_jobs + 2) * sizeof(int));  // and the counter
     const size_t total = s_tasks + s_start;
     if (ctx->plan_pinned.ensure(total) != ER_OK)
         return fail(ER_ERR_NOMEM, "batch: pinned staging failed");
@@ -1010,12 +1026,14 @@ int plan_create(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode, bool
         if (acc > INT32_MAX) return fail(ER_ERR_LIMIT, "batch: more than 2^31 bricks");
     }
     hs[n_jobs] = (int)acc;
+    hs[n_jobs + 1] = 0;
     p->n_items = (int)acc;
     if (pool_alloc(ctx, &p->d_block, total) != ER_OK)
         return fail(ER_ERR_NOMEM, "batch: device allocation failed");
     p->d_tasks = (GridTask*)p->d_block;
     p->d_start = (int*)((char*)p->d_block + s_tasks);
-    if (cudaMemcpyAsync(p->d_block, h, s_tasks + s_start, cudaMemcpyHostToDevice, ctx->stream) !=
+    p->d_head = (unsigned*)(p->d_start + n_jobs + 1);
+    if (cudaMemcpyAsync(p->d_block, h, total, cudaMemcpyHostToDevice, ctx->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         cudaGetLastError();
@@ -1157,8 +1175,8 @@ int er_grid_batch(er_ctx* ctx, const er_grid_job* jobs, int n_jobs, int mode) {
         int* d_left = (int*)ctx->task_left.ptr;
         ER_CUDA(ctx, cudaMemcpyAsync(d_left, left.data(), (size_t)n_jobs * sizeof(int),
                                      cudaMemcpyHostToDevice, ctx->stream));
-        st = launch_grid_batch(ctx, p->d_tasks, p->d_start, n_jobs, p->n_items, p->prec, d_left,
-                               ctx->done_dev);
+        st = launch_grid_batch(ctx, p->d_tasks, p->d_start, n_jobs, p->n_items, p->d_head, p->prec,
+                               d_left, ctx->done_dev);
         if (st != ER_OK) return st;
         cudaEvent_t fin;
         ER_CUDA(ctx, cudaEventCreateWithFlags(&fin, cudaEventDisableTiming));

@@ -22,3 +22,25 @@ def test_split_bricks_keep_the_bits(ctx, dims, comp):
     assert np.array_equal(single, out.cpu().numpy())
     fw.release()
 
+
+
+@pytest.mark.parametrize("n_jobs, dims", [(1, (86, 67, 35)), (3, (19, 40, 33)), (5, (2, 3, 2)), (2, (60, 64, 66))])
+def test_small_plans_replay(ctx, n_jobs, dims):
+    """Launches whose bricks all fit on the GPU are handed out by a counter that each
+    replay leaves as it found it: every replay writes every point (the last case has
+    too many bricks for that)."""
+    import torch
+    f = synth.make_framework(7, (17.0, 21.0, 19.0), (70.0, 101.0, 95.0), 200)
+    fw = ctx.upload(f.particles(), f.t_matrix, f.rep, f.rc2)
+    single = ctx.grid(fw, dims)
+    outs = [torch.empty(dims, dtype=torch.float32, device="cuda") for _ in range(n_jobs)]
+    plan = ctx.batch_plan([(fw, dims, o.data_ptr()) for o in outs], er.ER_BATCH_PERSISTENT)
+    for _ in range(3):
+        for o in outs:
+            o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        plan.run()
+        ctx.synchronize()
+        assert all(np.array_equal(o.cpu().numpy(), single) for o in outs)
+    plan.close()
+    fw.release()
